@@ -9,7 +9,7 @@
 //   3. k_sel_write   per listed row: (index, D, u, v) at its offset, so each
 //                    projection's points are in ascending index order, the
 //                    order of find()
-//   4. k_dft         F_j = sum_b E_v(j,b) sum_a E_u(j,a) P(a,b) per point
+//   4. k_dft_fold    F_j = sum_b E_v(j,b) sum_a E_u(j,a) P(a,b) per point
 //                    (k_dft_tcgen05 in grid_mma.cu for MIXED / FP16_SCALED)
 //   5. k_fill_grid   the output grid's zero pattern (CentroSymmetricity's
 //                    -0 imaginary parts on the mirrored half)
@@ -436,8 +436,7 @@ __global__ void __launch_bounds__(kSelThreads) k_sel_write_long(const ProjGeom *
 // ===========================================================================
 // exp(-2 pi i a w / n) with the phase reduced in FP64: a*w is exact (w is
 // FP32, |a| < 2^20), r = frac(a*w/n) in [-1/2, 1/2].
-template <typename T> __device__ __forceinline__ cplx<T> phase(int a, float w, double inv_n);
-template <> __device__ __forceinline__ double2 phase<double>(int a, float w, double inv_n)
+__device__ __forceinline__ double2 phase(int a, float w, double inv_n)
 {
     double t = (double)a * (double)w * inv_n;
     t -= rint(t);
@@ -445,19 +444,82 @@ template <> __device__ __forceinline__ double2 phase<double>(int a, float w, dou
     sincospi(-2.0 * t, &s, &c);
     return make_double2(c, s);
 }
-template <> __device__ __forceinline__ float2 phase<float>(int a, float w, double inv_n)
+
+// The FP64 DFT, folded on both axes.  With a, b counted from the projection's
+// centre, theta = 2 pi u / n1 and phi = 2 pi v / n2, the pairs (a, -a) and
+// (b, -b) share cosines and sines:
+//   F = sum_b (cos phi b - i sin phi b) (C(b) - i S(b)),
+//   C(b) = sum_{a >= 0} cos(theta a) Pe(a, b),  S(b) = sum_{a > 0} sin(theta a) Po(a, b),
+//   Pe(a, b) = P(a, b) + P(-a, b),  Po(a, b) = P(a, b) - P(-a, b),
+// and C and S are folded over b the same way.  A point then takes D1 D2 real
+// multiply-adds instead of 2 D1 D2.
+//
+// Bound: the FP64 pipe (2 multiply-adds per clock per SM: 0.53 ms for the
+// first case below).  Kernel times, unfolded with one sincospi per point, row
+// and column -> here:
+//   64 x 64, 31 projections, 81 k points       5.16 -> 0.77 ms
+//   128 x 128, 60 projections, 456 k points    56.4 -> 13.8 ms
+//   256 x 256, 90 projections, 2.77 M points   680 -> 309 ms
+//
+// k_fold_projections stores, per projection, column slot and a = 0 .. m1, the
+// four values (g0, g1, g2, g3) that a point multiplies by (cos, cos, sin, sin):
+//   slot b > 0:  Pe(a, b) +- Pe(a, -b),  Po(a, b) +- Po(a, -b)
+//   slot 0:      Pe(a, 0), Pe(a, -D2/2), Po(a, 0), Po(a, -D2/2)
+// For an even D2 the column -D2/2 has no partner and rides in slot 0, whose
+// column 0 needs half of the sums; so there are D2/2 slots (even) or
+// (D2 + 1) / 2 (odd, -D2/2 then being a regular column and absent from slot 0).
+constexpr int kFoldSlots = 8;     // column slots of a warp's register tile
+constexpr int kFoldPts = 32;      // points per CTA, one per lane
+constexpr int kFoldA = 128;       // rows a of one shared-memory table of phases
+constexpr int kFoldWarps = 4;
+
+struct FoldShape {
+    int D1, D2, m1, m2, nslots, nslots_p;  // nslots_p: rounded up to kFoldSlots (zero slots)
+};
+static FoldShape fold_shape(int D1, int D2)
 {
-    double t = (double)a * (double)w * inv_n;
-    t -= rint(t);
-    float s, c;
-    sincospif((float)(-2.0 * t), &s, &c);
-    return make_float2(c, s);
+    FoldShape f;
+    f.D1 = D1; f.D2 = D2;
+    f.m1 = D1 / 2; f.m2 = D2 / 2;
+    f.nslots = (D2 % 2 == 0) ? D2 / 2 : (D2 + 1) / 2;
+    f.nslots_p = (f.nslots + kFoldSlots - 1) / kFoldSlots * kFoldSlots;
+    return f;
 }
 
-constexpr int kDftJ = 8;      // points per CTA (one warp each)
-constexpr int kDftA = 16;     // projection rows per shared-memory chunk
-constexpr int kDftB = 256;    // projection columns per pass (8 per lane)
-constexpr int kDftPitch = kDftB + 1;
+// Grid: x over a, y = slot, z = projection (grid-stride).
+__global__ void __launch_bounds__(128) k_fold_projections(const double *__restrict__ proj, FoldShape f, int P,
+                                                          double4_32a *__restrict__ G)
+{
+    const int a = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
+    if (a > f.m1) return;
+    for (int p = blockIdx.z; p < P; p += gridDim.z) {
+        const double *src = proj + (long long)p * f.D1 * f.D2;
+        auto at = [&](int x, int b) -> double {  // P(x, b), zero outside the projection
+            const int i = x + f.m1, j = b + f.m2;
+            return (i >= 0 && i < f.D1 && j >= 0 && j < f.D2) ? src[i + (long long)f.D1 * j] : 0.0;
+        };
+        auto pe = [&](int b) { return a == 0 ? at(0, b) : at(a, b) + at(-a, b); };
+        auto po = [&](int b) { return a == 0 ? 0.0 : at(a, b) - at(-a, b); };
+        double4_32a g;
+        g.x = g.y = g.z = g.w = 0.0;
+        if (s == 0) {
+            const bool half = f.D2 % 2 == 0;
+            g.x = pe(0);
+            g.z = po(0);
+            if (half) {
+                g.y = pe(-f.m2);
+                g.w = po(-f.m2);
+            }
+        } else if (s < f.nslots) {
+            const double e0 = pe(s), e1 = pe(-s), o0 = po(s), o1 = po(-s);
+            g.x = e0 + e1;
+            g.y = e0 - e1;
+            g.z = o0 + o1;
+            g.w = o0 - o1;
+        }
+        G[((long long)p * f.nslots_p + s) * (f.m1 + 1) + a] = g;
+    }
+}
 
 struct DftTile {
     int proj;
@@ -465,66 +527,102 @@ struct DftTile {
     long long j0;
 };
 
-// One CTA: kDftJ points of one projection.  Warp w owns point j0 + w and
-// accumulates Q(b) = sum_a E_u(a) P(a,b) for its lane's 8 columns b, then
-// contracts with E_v(b) and reduces across the warp.
-template <typename T>
-__global__ void __launch_bounds__(256) k_dft(const T *__restrict__ proj, int D1, int D2, int n1, int n2,
-                                            const DftTile *__restrict__ tiles, const float *__restrict__ uu,
-                                            const float *__restrict__ vv, cplx<T> *__restrict__ F)
+// One CTA: kFoldPts points of one projection, a lane per point; the warps take
+// tiles of kFoldSlots column slots in turn (rotated by the block index, so
+// that a tile count that is no multiple of the warps loads the four schedulers
+// alike).  The values of G are the same for all lanes: each load is one
+// broadcast, and there are two 32-byte loads per four multiply-adds.  The
+// phases E(a) = E(8 s) E(r), r < 8, take one rounding of a complex product on
+// top of sincospi's, and are shared by the warps through a table of kFoldA
+// rows (made again per round of slot tiles when D1 is larger than that).
+__global__ void __launch_bounds__(32 * kFoldWarps) k_dft_fold(const double4_32a *__restrict__ G, FoldShape f, int n1,
+                                                             int n2, const DftTile *__restrict__ tiles,
+                                                             const float *__restrict__ uu,
+                                                             const float *__restrict__ vv, double2 *__restrict__ F)
 {
-    __shared__ T Ps[kDftA * kDftPitch];
-    __shared__ cplx<T> Eu[kDftJ * kDftA];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2 *E = reinterpret_cast<double2 *>(smem_raw);         // [rows of the chunk][kFoldPts]: E_u(a)
+    __shared__ double2 Ru[8][kFoldPts], Rv[8][kFoldPts];        // E_u(r), E_v(r)
+    __shared__ double2 part[kFoldWarps][kFoldPts];
     const DftTile tl = tiles[blockIdx.x];
-    const T *P = proj + (long long)tl.proj * D1 * D2;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int amin = -(D1 / 2), bmin = -(D2 / 2);
     const double inv1 = 1.0 / (double)n1, inv2 = 1.0 / (double)n2;
-    const bool active = w < tl.nj;
-    const float my_v = active ? vv[tl.j0 + w] : 0.f;
-    cplx<T> acc = mk((T)0, (T)0);
-    for (int b0 = 0; b0 < D2; b0 += kDftB) {
-        const int nb = min(kDftB, D2 - b0);
-        cplx<T> q[kDftB / 32];
+    const bool active = lane < tl.nj;
+    const float u = active ? uu[tl.j0 + lane] : 0.f, v = active ? vv[tl.j0 + lane] : 0.f;
+    for (int r = w; r < 16; r += kFoldWarps) {
+        if (r < 8) Ru[r][lane] = phase(r, u, inv1);
+        else Rv[r - 8][lane] = phase(r - 8, v, inv2);
+    }
+    const int ntile = f.nslots_p / kFoldSlots;
+    const int rounds = (ntile + kFoldWarps - 1) / kFoldWarps;
+    const int nchunk = (f.m1 + kFoldA - 1) / kFoldA;
+    const int rw = (w + blockIdx.x) % kFoldWarps;
+    double fx = 0.0, fy = 0.0;
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int tile = rd * kFoldWarps + rw;
+        const bool on = tile < ntile;
+        const double4_32a *Gt = G + ((long long)tl.proj * f.nslots_p + (on ? tile : 0) * kFoldSlots) * (f.m1 + 1);
+        double acc[kFoldSlots][4];
+        for (int ch = 0; ch < nchunk; ++ch) {
+            const int a0 = 1 + ch * kFoldA, na = min(kFoldA, f.m1 + 1 - a0);
+            if (rd == 0 || nchunk > 1) {
+                __syncthreads();  // Ru is written, and the table's last readers are done
+                for (int g = w; 8 * g < na; g += kFoldWarps) {
+                    const double2 h = phase(a0 + 8 * g, u, inv1);
 #pragma unroll
-        for (int m = 0; m < kDftB / 32; ++m) q[m] = mk((T)0, (T)0);
-        for (int a0 = 0; a0 < D1; a0 += kDftA) {
-            const int na = min(kDftA, D1 - a0);
-            __syncthreads();
-            for (int idx = threadIdx.x; idx < kDftA * kDftB; idx += blockDim.x) {
-                const int a = idx % kDftA, b = idx / kDftA;
-                Ps[a * kDftPitch + b] = (a < na && b < nb) ? P[(a0 + a) + (long long)D1 * (b0 + b)] : (T)0;
+                    for (int r = 0; r < 8; ++r)
+                        if (8 * g + r < na) E[(8 * g + r) * kFoldPts + lane] = r ? cmul(h, Ru[r][lane]) : h;
+                }
+                __syncthreads();
             }
-            if (threadIdx.x < kDftJ * kDftA) {
-                const int j = threadIdx.x / kDftA, a = threadIdx.x % kDftA;
-                Eu[threadIdx.x] = (j < tl.nj && a < na) ? phase<T>(amin + a0 + a, uu[tl.j0 + j], inv1)
-                                                        : mk((T)0, (T)0);
+            if (!on) continue;
+            if (ch == 0) {  // a = 0: the cosine is 1, the sine 0
+#pragma unroll
+                for (int s = 0; s < kFoldSlots; ++s) {
+                    const double4_32a g = Gt[(long long)s * (f.m1 + 1)];
+                    acc[s][0] = g.x;
+                    acc[s][1] = g.y;
+                    acc[s][2] = acc[s][3] = 0.0;
+                }
             }
-            __syncthreads();
             for (int a = 0; a < na; ++a) {
-                const cplx<T> e = Eu[w * kDftA + a];
+                const double2 e = E[a * kFoldPts + lane];  // (cos, -sin)
 #pragma unroll
-                for (int m = 0; m < kDftB / 32; ++m) {
-                    const T pv = Ps[a * kDftPitch + lane + 32 * m];
-                    q[m].x += e.x * pv;
-                    q[m].y += e.y * pv;
+                for (int s = 0; s < kFoldSlots; ++s) {
+                    const double4_32a g = Gt[(long long)s * (f.m1 + 1) + a0 + a];
+                    acc[s][0] = fma(e.x, g.x, acc[s][0]);
+                    acc[s][1] = fma(e.x, g.y, acc[s][1]);
+                    acc[s][2] = fma(e.y, g.z, acc[s][2]);  // -S
+                    acc[s][3] = fma(e.y, g.w, acc[s][3]);
                 }
             }
         }
-        if (active) {
+        if (!on) continue;
+        // contraction with E_v: (C + i acc2) (ev.x + i ev.y) per slot, folded over b
+        const double2 h = phase(tile * kFoldSlots, v, inv2);
 #pragma unroll
-            for (int m = 0; m < kDftB / 32; ++m) {
-                const int b = lane + 32 * m;
-                if (b < nb) acc = cadd(acc, cmul(q[m], phase<T>(bmin + b0 + b, my_v, inv2)));
+        for (int s = 0; s < kFoldSlots; ++s) {
+            if (tile == 0 && s == 0) {
+                const double2 em = phase(-f.m2, v, inv2);
+                fx += acc[0][0] + (em.x * acc[0][1] - em.y * acc[0][3]);
+                fy += acc[0][2] + (em.x * acc[0][3] + em.y * acc[0][1]);
+            } else {
+                const double2 ev = s ? cmul(h, Rv[s][lane]) : h;
+                fx += ev.x * acc[s][0] - ev.y * acc[s][3];
+                fy += ev.x * acc[s][2] + ev.y * acc[s][1];
             }
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        acc.x += __shfl_down_sync(0xffffffffu, acc.x, o);
-        acc.y += __shfl_down_sync(0xffffffffu, acc.y, o);
+    part[w][lane] = make_double2(fx, fy);
+    __syncthreads();
+    if (w == 0 && active) {
+        double2 t = part[0][lane];
+        for (int k = 1; k < kFoldWarps; ++k) {
+            t.x += part[k][lane].x;
+            t.y += part[k][lane].y;
+        }
+        F[tl.j0 + lane] = t;
     }
-    if (active && lane == 0) F[tl.j0 + w] = acc;
 }
 
 // ===========================================================================
@@ -918,19 +1016,27 @@ static void grid_dft_t(genfire_ctx *ctx, const genfire_params &p, const double *
                     sel.v.as<float>(), reinterpret_cast<float2 *>(F.p), dft_err.as<int>(), se.event(6), se.event(7),
                     p.precision == GENFIRE_PREC_FP16_SCALED);
     } else {
-        // FP64: kDftJ consecutive points of one projection per CTA
+        // FP64: the folded projections, then kFoldPts consecutive points of one projection per CTA
         std::vector<DftTile> tiles;
-        tiles.reserve((size_t)(sel.total / kDftJ + P));
+        tiles.reserve((size_t)(sel.total / kFoldPts + P));
         for (int i = 0; i < P; ++i)
-            for (long long j = 0; j < sel.nk[i]; j += kDftJ)
-                tiles.push_back(DftTile{i, (int)std::min<long long>(kDftJ, sel.nk[i] - j), sel.off[i] + j});
+            for (long long j = 0; j < sel.nk[i]; j += kFoldPts)
+                tiles.push_back(DftTile{i, (int)std::min<long long>(kFoldPts, sel.nk[i] - j), sel.off[i] + j});
         if (!tiles.empty()) {
+            const FoldShape f = fold_shape(D1, D2);
             DevBuf dt(sizeof(DftTile) * tiles.size(), st);
+            DevBuf G(sizeof(double4_32a) * (size_t)P * f.nslots_p * (f.m1 + 1), st);
             GF_CUDA(cudaMemcpyAsync(dt.p, tiles.data(), sizeof(DftTile) * tiles.size(), cudaMemcpyHostToDevice, st));
+            k_fold_projections<<<dim3(cdiv(f.m1 + 1, 128), f.nslots_p, std::min(P, 65535)), 128, 0, st>>>(
+                d_proj, f, P, G.as<double4_32a>());
+            GF_CHECK_LAUNCH();
+            const size_t smem = sizeof(double2) * kFoldPts * std::min(f.m1, kFoldA);
+            GF_CUDA(cudaFuncSetAttribute((const void *)k_dft_fold, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(sizeof(double2) * kFoldPts * kFoldA)));
             se.mark(6, st);
-            k_dft<double><<<(unsigned)tiles.size(), 256, 0, st>>>(d_proj, D1, D2, n1, n2, dt.as<DftTile>(),
-                                                                   sel.u.as<float>(), sel.v.as<float>(),
-                                                                   reinterpret_cast<double2 *>(F.p));
+            k_dft_fold<<<(unsigned)tiles.size(), 32 * kFoldWarps, smem, st>>>(
+                G.as<double4_32a>(), f, n1, n2, dt.as<DftTile>(), sel.u.as<float>(), sel.v.as<float>(),
+                reinterpret_cast<double2 *>(F.p));
             GF_CHECK_LAUNCH();
             se.mark(7, st);
         }
