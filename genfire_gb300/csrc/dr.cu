@@ -25,6 +25,7 @@
 #include "fft.cuh"
 #include "fft_reg.cuh"
 #include "fft_r32.cuh"
+#include "fft_two.cuh"
 #include "internal.h"
 
 #include <algorithm>
@@ -124,11 +125,12 @@ template <typename T, int N> static void set_reg_attrs()
 // float columns per thread (unit column stride and 16-byte aligned column
 // pairs: even strides, aligned bases; tiles start at even columns), the
 // mixed-radix engine, the radix-32 engines for 512 and 1024 complex64 points
-// (fft_r32.cuh: 32 x 16 and 32 x 32, one exchange per transform), and for the
+// (fft_r32.cuh: 32 x 16 and 32 x 32, one exchange per transform), the two-stage
+// engine for lengths that split into two factors up to 32, and for the
 // fused 512-point pass the persistent radix-32 pass fed by TMA tensor copies
 // (measured 6 % slower than variant 4 on the 512^3 iteration; an autotuner
 // candidate).
-enum ColVariant { kColAuto = -1, kColGeneric = 0, kColReg1 = 1, kColReg2 = 2, kColMix = 3, kColR32 = 4, kColR32Tma = 5 };
+enum ColVariant { kColAuto = -1, kColGeneric = 0, kColReg1 = 1, kColReg2 = 2, kColMix = 3, kColR32 = 4, kColR32Tma = 5, kColTwo = 6 };
 
 // GENFIRE_COL_VARIANT=<v> forces variant v wherever it is valid (tuning and
 // tests); unset, the built-in choice or the autotuner decides
@@ -296,6 +298,7 @@ template <typename T> static bool col_variant_ok(const ColPassArgs<T> &a, int v,
     if (v == kColR32)
         return sizeof(T) == 4 && r32_width(a.pl.n) > 0 && span_ok(a) && (!(a.mode & 4) || a.W == r32_width(a.pl.n));
     if (v == kColMix) return span_ok(a) && mix_capable<T>(a.pl.n);
+    if (v == kColTwo) return span_ok(a) && two_capable<T>(a.pl.n);
     if (!reg_capable(a)) return false;
     return v == kColReg1 || (v == kColReg2 && pair_capable(a));
 }
@@ -306,8 +309,10 @@ template <typename T> static bool col_variant_ok(const ColPassArgs<T> &a, int v,
 // powers of two, two columns per thread in the fused forward + constraint +
 // inverse pass (two transforms per load) and one column per thread in the
 // single-transform passes (twice the resident warps); the mixed-radix
-// register engine for 3 or 5 times a power of two; the generic engine for
-// other lengths.
+// register engine for 3 or 5 times a power of two (the two-stage engine is
+// within 15 % of it either way there, and a candidate of the autotuner); the
+// two-stage engine for the other lengths that split (450 points, the fused
+// pass: 2.21 ms generic, 0.33 ms); the generic engine for the rest.
 template <typename T> static int default_col_variant(const ColPassArgs<T> &a)
 {
     // below 512 points the radix-32 engine is a candidate of the autotuner, not
@@ -316,6 +321,7 @@ template <typename T> static int default_col_variant(const ColPassArgs<T> &a)
     if (a.pl.n >= 512 && col_variant_ok(a, kColR32)) return kColR32;
     if (reg_capable(a)) return ((a.mode & 3) == 3 && pair_capable(a)) ? kColReg2 : kColReg1;
     if (col_variant_ok(a, kColMix)) return kColMix;
+    if (col_variant_ok(a, kColTwo)) return kColTwo;
     return kColGeneric;
 }
 
@@ -389,6 +395,8 @@ template <typename T> static void launch_colpass(ColPassArgs<T> a, int other, cu
         }
     } else if (variant == kColMix) {
         if (!launch_col_mix<T>(a, other, st)) fail(GENFIRE_ERR_STATE, "internal: mixed-radix pass not available.");
+    } else if (variant == kColTwo) {
+        if (!launch_col_two<T>(a, other, st)) fail(GENFIRE_ERR_STATE, "internal: two-stage pass not available.");
     } else if (variant == kColGeneric) {
         const size_t sm = tile_smem<T>(a.pl.n, a.W);
         dim3 grid(cdiv(a.ncols, a.W), other);
@@ -430,7 +438,7 @@ template <typename T> static int autotune_colpass(ColPassArgs<T> a, int other, c
     // (keeps the choice stable against timing noise)
     int best = kColAuto;
     float best_ms = 0, default_ms = -1;
-    for (int v : {kColGeneric, kColReg1, kColReg2, kColMix, kColR32, kColR32Tma}) {
+    for (int v : {kColGeneric, kColReg1, kColReg2, kColMix, kColR32, kColR32Tma, kColTwo}) {
         if (!col_variant_ok(a, v, other)) continue;
         launch_colpass<T>(a, other, st, v);
         GF_CUDA(cudaEventRecord(e0, st));
@@ -469,7 +477,17 @@ template <typename T> static void launch_rows(RowPassArgs<T> a, bool forward, cu
             return;
         }
     }
-    if (!try_rows_reg<T>(a, forward, st) && !launch_rows_mix<T>(a, forward, st)) {
+    // complex64 lengths with two-stage kernels of their own take them before the
+    // mixed-radix engine (F1 + I1 per iteration: 192 points 21.5 -> 18.2 us, 320
+    // points 50.7 -> 36.0 us, 384 points 59.8 -> 53.0 us); complex128 is bound by
+    // its arithmetic either way and keeps the mixed-radix passes
+    if constexpr (sizeof(T) == 4) {
+        if (two_fixed(a.pl.n) && launch_rows_two<T>(a, forward, st)) {
+            GF_CHECK_LAUNCH();
+            return;
+        }
+    }
+    if (!try_rows_reg<T>(a, forward, st) && !launch_rows_mix<T>(a, forward, st) && !launch_rows_two<T>(a, forward, st)) {
         const size_t sm = tile_smem<T>(a.pl.n, a.W);
         const int pairs = (a.nrows + 1) / 2;
         dim3 grid(cdiv(pairs, a.W));
@@ -497,6 +515,14 @@ __global__ void k_half_from_centered(const cplx<T> *__restrict__ M, int n1, int 
         const cplx<T> x = M[ra + (q1 + n1 / 2) % n1], y = M[rb + (m1 + n1 / 2) % n1];
         H[q1 + (long long)ld1 * (q2 + (long long)n2 * q3)] = mk((T)0.5 * (x.x + y.x), (T)0.5 * (x.y - y.y));
     }
+}
+
+// 1 / N as a value and the rest of it, less the mean gain of the transforms
+template <typename T> static void inverse_scale(RowPassArgs<T> &r, double N, double gain)
+{
+    const double s = (1.0 - gain) / N;
+    r.scale = (T)(1.0 / N);
+    r.scale_lo = (T)(s - (double)r.scale);
 }
 
 static int round_up(int a, int b) { return (a + b - 1) / b * b; }
@@ -556,7 +582,7 @@ static void rec_ifft_t(genfire_ctx *ctx, const cplx<T> *d_M, int n1, int n2, int
     std::memset(&r, 0, sizeof(r));
     r.pl = c.pl1; r.tw = c.tw1; r.W = c.W1; r.nrows = D2 * D1; r.B1 = D1; r.c1 = D1 / 2; r.h1 = c.h1; r.ld1 = c.ld1;
     r.xs[0] = d_rec; r.xsel = nullptr; r.Y = Z.as<cplx<T>>();
-    r.scale = (T)(1.0 / ((double)n1 * n2 * n1));
+    inverse_scale<T>(r, (double)n1 * n2 * n1, 0.0);
     launch_rows<T>(r, false, st);
 }
 
@@ -1256,6 +1282,26 @@ template <typename T> struct ReconT : ReconBase {
         GF_CUDA(cudaStreamSynchronize(st));
     }
 
+    // the mean gain of the iteration's forward and inverse transforms, where they
+    // run on the two-stage engine (two_gain; the other engines' is left as it is)
+    double transform_gain() const
+    {
+        if constexpr (sizeof(T) == 8) return 0.0;
+        auto column = [](ColPassArgs<T> a, int v) {  // the engine launch_colpass takes for a pass
+            const int f = forced_col_variant();
+            if (f != kColAuto && col_variant_ok(a, f)) v = f;
+            if (v == kColAuto || !col_variant_ok(a, v)) v = default_col_variant(a);
+            return v == kColTwo;
+        };
+        ReconT *self = const_cast<ReconT *>(this);
+        double g = 0;
+        if (two_fixed(n1)) g += two_gain(n1);
+        if (column(self->f2_args(), vF2)) g += 0.5 * two_gain(n2);
+        if (column(self->i2_args(false), vI2)) g += 0.5 * two_gain(n2);
+        if (column(self->f3_args(), vF3)) g += two_gain(n1);
+        return g;
+    }
+
     // ev (optional) receives an event before each of the 7 kernels and one after
     void enqueue_iteration(cudaStream_t st, cudaEvent_t *ev = nullptr)
     {
@@ -1300,7 +1346,7 @@ template <typename T> struct ReconT : ReconBase {
         // every row is written
         q.pairmask = p.monitor_R == 1 ? nullptr : pairmask.as<uint8_t>();
         q.positivity = 0;
-        q.scale = (T)(1.0 / ((double)n1 * n2 * n1));
+        inverse_scale<T>(q, (double)n1 * n2 * n1, transform_gain());
         launch_rows<T>(q, false, st);
         mark();
     }

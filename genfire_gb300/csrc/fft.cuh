@@ -596,6 +596,7 @@ template <typename T> struct RowPassArgs {
     int positivity;
     cplx<T> *Y;        // ld1 x nrows half spectrum
     T scale;           // inverse only
+    T scale_lo;        // what scale misses of the exact factor (two-stage passes; 0 elsewhere)
     // with ctl set (the iteration's first pass): CTA 0 starts the iteration
     // (ctl_begin_update) while every CTA reads the object from xs[ctl->xnext]
     Ctl *ctl;

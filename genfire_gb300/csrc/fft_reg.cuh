@@ -203,9 +203,11 @@ __device__ __forceinline__ void reg_fft(cplx<T> (&v)[NC][8], cplx<T> *sA, cplx<T
 template <typename T> using ErrAcc = typename std::conditional<sizeof(T) == 8, double, float>::type;
 
 // Fourier constraint and errK terms on one shared-memory tile (see k_colpass);
-// returns this thread's errK terms.
-template <typename T, class Lay>
-__device__ __forceinline__ ErrAcc<T> apply_table(cplx<T> *s, const ColPassArgs<T> &a, int tile, int W, int other)
+// returns this thread's errK terms; idx maps (q3, column in tile) to the
+// tile's shared-memory slot.
+template <typename T, class Idx>
+__device__ __forceinline__ ErrAcc<T> apply_table_at(cplx<T> *s, const ColPassArgs<T> &a, int tile, int W, int other,
+                                                    Idx idx)
 {
     using A_ = ErrAcc<T>;
     const int cid0 = other * a.h1 + tile * W;
@@ -216,7 +218,7 @@ __device__ __forceinline__ ErrAcc<T> apply_table(cplx<T> *s, const ColPassArgs<T
     for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
         const TabEntry<T> t = a.tab[e];
         const int q3 = t.pos & 0xFFFF, cl = t.pos >> 16;
-        const int si = Lay::idx(q3, cl);
+        const int si = idx(q3, cl);
         const cplx<T> k = s[si];
         const A_ mk_ = (A_)sqrt(k.x * k.x + k.y * k.y);
         if (t.eflags & 1u) acc += fabs(mk_ - (A_)sqrt(t.Mq.x * t.Mq.x + t.Mq.y * t.Mq.y));
@@ -229,6 +231,11 @@ __device__ __forceinline__ ErrAcc<T> apply_table(cplx<T> *s, const ColPassArgs<T
         }
     }
     return acc;
+}
+template <typename T, class Lay>
+__device__ __forceinline__ ErrAcc<T> apply_table(cplx<T> *s, const ColPassArgs<T> &a, int tile, int W, int other)
+{
+    return apply_table_at<T>(s, a, tile, W, other, [](int q3, int cl) { return Lay::idx(q3, cl); });
 }
 
 // CTA sum of the per-thread errK terms: warp sums in FP32 (a few terms per
