@@ -212,6 +212,11 @@ constexpr int r32_col_min_blocks(int n) { return n == 512 ? 5 : n == 1024 ? 4 : 
 // with it, so they do without.
 constexpr int r32_prefetch_ahead(int n, bool fused) { return (n == 512 && !fused) ? 380 : 0; }
 
+// Only where a tile's rows lie near each other (a pass along dim 2: rows ld1
+// elements apart).  Along dim 3 a row is a megabyte from the next, and the
+// prefetch cost the inverse pass of a 512^3 recIFFT 30 % (301 us, 231 without).
+constexpr long long kR32PrefetchSpan = 1 << 14;  // elements between rows
+
 // The transforms, the table phase and the stores of one tile (tile, other)
 // of a column pass whose input is already in x (slot m holds element t + P m);
 // tiles_x is the number of tiles along the columns (the index of the tile's
@@ -310,7 +315,7 @@ __global__ void __launch_bounds__(R32<N>::THREADS, r32_col_min_blocks(N)) k_col_
         // kernel reads itself (column 0 of a valid tile, r < in_cnt)
         const long long nb = (long long)gridDim.x * gridDim.y;
         const long long fb = (long long)blockIdx.y * gridDim.x + blockIdx.x + r32_prefetch_ahead(N, ZIN && ZOUT);
-        if (fb < nb && a.col_stride == 1) {
+        if (fb < nb && a.col_stride == 1 && a.in_dim < kR32PrefetchSpan) {
             const int ftile = (int)(fb % gridDim.x), fother = (int)(fb / gridDim.x);
             const cplx<T> *fin = a.in + (long long)fother * a.in_other + (long long)ftile * W;
             for (int r = threadIdx.x; r < a.in_cnt; r += G::THREADS)
