@@ -4,20 +4,34 @@
 // For one projection P (D1 x D2) and a tile of 128 selected K-points j:
 //   Q(j, b) = sum_a E_u(j, a) P(a, b),  E_u(j, a) = exp(-2 pi i a u_j / n1)
 //   F_j     = sum_b Q(j, b) E_v(j, b),  E_v(j, b) = exp(-2 pi i b v_j / n2)
-// (fillInFourierGrid_DFT.m:243).  Q is a GEMM with M = 128 K-points, N = D2
-// and K = D1.  Operands are split into hi + lo parts of a 16-bit type and
-// multiplied as hi*hi + hi*lo + lo*hi with FP32 accumulation:
-//   Re Q += Re(E_u)_hi P_hi + Re(E_u)_hi P_lo + Re(E_u)_lo P_hi
-//   Im Q += Im(E_u)_hi P_hi + Im(E_u)_hi P_lo + Im(E_u)_lo P_hi
+// (fillInFourierGrid_DFT.m:243).  P is real and E_u(-a) = conj E_u(a), so the
+// rows fold in pairs (a counted from the projection's centre):
+//   Re Q(j, b) = P(0, b) + sum_{a > 0} Re E_u(j, a) Pe(a, b),  Pe(a, b) = P(a, b) + P(-a, b)
+//   Im Q(j, b) =           sum_{a > 0} Im E_u(j, a) Po(a, b),  Po(a, b) = P(a, b) - P(-a, b)
+// (the row -D1/2 of an even D1 has no partner: P(D1/2, b) counts as zero).
+// Each is a GEMM with M = 128 K-points, N = D2 and K = D1/2: half the matrix
+// products of the unfolded form, whose two GEMMs share P and have K = D1.  The
+// row a = 0 is added in the epilogue.  Operands are split into hi + lo parts of a
+// 16-bit type and multiplied as hi*hi + hi*lo + lo*hi with FP32 accumulation:
+//   Re Q += Re(E_u)_hi Pe_hi + Re(E_u)_hi Pe_lo + Re(E_u)_lo Pe_hi
+//   Im Q += Im(E_u)_hi Po_hi + Im(E_u)_hi Po_lo + Im(E_u)_lo Po_hi
 // The 16-bit type is BF16 (GENFIRE_PREC_MIXED: ~16 significant bits per
 // operand) or FP16 (GENFIRE_PREC_FP16_SCALED: ~22 bits, with each projection
-// scaled by a power of two so that its largest value sits just below 2^14 and
-// the lo parts stay in FP16's normal range; the scale is undone exactly in the
-// epilogue).
+// scaled by a power of two so that its largest value sits just below 2^14, its
+// folded ones below 2^15, and the lo parts stay in FP16's normal range; the
+// scale is undone exactly in the epilogue).
 //
-// Work decomposition.  P is pre-split once into blocks of 128 columns (b) by
-// 256 rows (a) in the canonical no-swizzle K-major layout (128 KB per block,
-// hi and lo).  A unit of work is (tile of 128 points, block): the tile's
+// DFT kernel, unfolded -> here: 256 x 256, 90 projections, 2.77 M points 1.586 ->
+// 0.818 ms (0.47 of the measured bf16 rate in useful products, 0.71 in executed
+// ones); 128 x 128, 60 projections 0.085 -> 0.056; 150 x 105 on a 450 x 315 grid,
+// 40 projections, FP16 0.365 -> 0.181; 512 x 512, 120 projections 34.7 -> 16.9.
+// With the fold alone it took 0.996 ms on the first: 70 cycles per MMA and 2,500
+// per unit, which the issue thread's own instructions (0.96 -> 0.90) and the
+// second groups of producer and epilogue warps (0.90 -> 0.82) took out.
+//
+// Work decomposition.  P is folded and pre-split once into blocks of 128 columns
+// (b) by 128 folded rows (a) in the canonical no-swizzle K-major layout (128 KB
+// per block: Pe and Po, hi and lo).  A unit of work is (tile of 128 points, block): the tile's
 // partial Q over the block's rows and columns, contracted with E_v over the
 // block's columns, gives a partial F; the partials of a point (one per block
 // of its projection, two for 256 x 256 projections) are summed in block order
@@ -27,21 +41,25 @@
 // only a few times.
 //
 // Warp roles in each CTA:
-//   warps 0-3   epilogue: thread = TMEM lane = point; tcgen05.ld of the Re and
-//               Im accumulators, per 16-column group Horner's rule in E_v(2)
-//               over its even and odd columns at once (packed FP32 pairs),
-//               times an anchor E_v(b_g) (exact every 64 columns), partial F
-//               stored;
-//   warp 4      one thread loads blocks (cp.async.bulk into shared memory,
+//   warps 0-7   epilogue, two groups of four, each the units of one accumulator
+//               buffer: thread = TMEM lane = point; tcgen05.ld of the Re and Im
+//               accumulators eight columns ahead, Horner's rule in E_v(2) over
+//               even and odd columns at once (packed FP32 pairs), times an anchor
+//               E_v(b_g) (exact every 64 columns), partial F stored;
+//   warp 8      one thread loads blocks (cp.async.bulk into shared memory,
 //               completing on an mbarrier) and issues tcgen05.mma (M = 128,
 //               N <= 128, K = 16), committing to mbarriers;
-//   warps 5-12  A producers: per 32-wide K chunk, each thread forms 16
-//               consecutive E_u(j, a) of one point as packed FP32 pairs
-//               (real parts of two neighbours in one register pair, imaginary
-//               parts in another) by four independent chains of packed
-//               rotations from an anchor (exact every 4 chunks), splits them
-//               into hi/lo (one packed subtraction per pair) and stores them in
-//               the K-major layout; three A stages.
+//   warps 9-16  A producers, two groups of four that take every other unit: per
+//               32-wide K chunk, each thread forms the 32 consecutive E_u(j, a) of
+//               one point, eight at a time, as packed FP32 pairs (real parts of
+//               two neighbours in one register pair, imaginary parts in another)
+//               by packed rotations from an anchor (exact at a block's first
+//               chunk), splits them into hi/lo (one packed subtraction per pair)
+//               and stores them in the K-major layout; three A stages.
+// Two groups each, because a unit begins with a chain of latencies (its point's
+// coordinate, then reduced phases with sine and cosine) and one warp per
+// scheduler cannot hide its own chains: one group's start runs beside the
+// other's work.  544 threads leave 96 registers, hence the eights.
 // The accumulator (Re and Im, 2 x 128 columns) is double buffered in TMEM, so
 // the epilogue of one unit overlaps the MMAs of the next.
 //
@@ -190,6 +208,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // exp(-2 pi i * a * w / n) for integer a and FP32 w, phase reduced in FP64
@@ -274,18 +299,19 @@ __device__ __forceinline__ float bf16_hi_f(uint32_t w) { return __uint_as_float(
 namespace umma {
 
 constexpr int kN = 128;                        // columns of one block (N of the MMAs)
-constexpr int kKR = 256;                       // rows of one block (its K range)
-constexpr int kKCB = kKR / kKC;                // K chunks per block (8)
+constexpr int kKR = 128;                       // folded rows of one block (its K range)
+constexpr int kKCB = kKR / kKC;                // K chunks per block (4)
 constexpr int kABytes = kM * kKC * 2;          // one A array of a chunk (8 KB)
 constexpr int kAStage = 4 * kABytes;           // re_hi, re_lo, im_hi, im_lo (32 KB)
 constexpr int kStages = 3;
 constexpr int kBArr = kN * kKC;                // elements of one B array of a chunk
-constexpr int kBChunk = 2 * kBArr * 2;         // hi + lo of one chunk (16 KB)
+constexpr int kBChunk = 4 * kBArr * 2;         // Pe and Po, hi and lo, of one chunk (32 KB)
 constexpr int kBBytes = kKCB * kBChunk;        // one block (128 KB)
-constexpr int kEpiWarps = 4, kMmaWarp = 4, kProdWarp0 = 5, kProdWarps = 8;
-constexpr int kProdThreads = 32 * kProdWarps;
-constexpr int kWsThreads = 32 * (kProdWarp0 + kProdWarps);  // 416
-constexpr int kNBars = 2 * kStages + 4 + 3;    // afull, aempty, tfull x2, tempty x2, bfull, bdone, drain
+constexpr int kEpiWarps = 4, kProdGroupWarps = 4;               // warps of one epilogue / producer group
+constexpr int kMmaWarp = 2 * kEpiWarps, kProdWarp0 = kMmaWarp + 1;
+constexpr int kProdGroupThreads = 32 * kProdGroupWarps;
+constexpr int kWsThreads = 32 * (kProdWarp0 + 2 * kProdGroupWarps);  // 544
+constexpr int kNBars = 2 * kStages + 4 + 3 + 2;  // afull, aempty, tfull x2, tempty x2, bfull, bdone, drain, handoff x2
 constexpr size_t kWsSmem = (size_t)kBBytes + kStages * kAStage + 8 * kNBars + 16;
 
 // kind::f16 instruction descriptor: FP32 accumulator, FP16 A and B, both K-major.
@@ -358,6 +384,12 @@ __device__ __forceinline__ f2x_t sub_x2(f2x_t a, f2x_t b)
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ f2x_t add_x2(f2x_t a, f2x_t b)
+{
+    f2x_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ f2x_t mul_x2(f2x_t a, f2x_t b)
 {
     f2x_t r;
@@ -391,30 +423,28 @@ template <bool F16> __device__ __forceinline__ void split_x2(f2x_t v, uint32_t &
 }  // namespace umma
 
 // One unit of work: a tile of up to 128 consecutive selected points of one
-// projection against one block (128 columns x 256 rows) of that projection.
+// projection against one block of that projection.
 struct WsUnit {
     long long j0;  // first point
     int proj;
     int blk;       // block index (proj * nnc + nc) * nkr + kr
     int nj;        // points in the tile (<= 128)
-    int pad;
+    int ncr;       // the block's column chunk nc | row block kr << 16
 };
 
 struct WsArgs {
-    const uint16_t *B;        // pre-split blocks: [blk][K chunk][hi|lo][128 x 32], 16-bit words
+    const uint16_t *B;        // pre-split blocks, 16-bit words: [blk][K chunk][Pe hi|Pe lo|Po hi|Po lo][128 x 32]
+                              // (second form: [hi|lo][256 x 32])
+    const float *P0;          // row a = 0 of each (scaled) projection, D2p values (first form)
     const WsUnit *units;
     int nunits;
     const float *u, *v;
     const float *inv_scale;   // per projection (1 for BF16)
     float2 *F;                // partial F: [part][ntot], part = nc * nkr + kr
     long long ntot;
-    int D1, D2, D1p, D2p;     // D1p: D1 rounded up to 32; D2p: D2 rounded up to 16
+    int D1, D2, Kp, D2p;      // Kp: K (D1/2 folded rows; second form: D1) rounded up to 32; D2p: D2 rounded up to 16
     int n1, n2, log2n1, log2n2;
     int nnc, nkr;
-    // first form, one K block of D1 = 64 H rows: K runs a = 0 .. 32H-1 (chunks
-    // 0 .. H-1) then a = -1 .. -32H (chunks H .. 2H-1), consumed as the pairs
-    // (p, H + p); 0 for the natural order
-    int mirror;
     int *err;                 // set to 1 when a bounded wait expired
     long long wait_cycles;    // limit of the pipeline's waits (the drain always allows kWaitCycles)
 };
@@ -428,19 +458,20 @@ __global__ void __launch_bounds__(umma::kWsThreads, 1) k_dft_tcgen05(WsArgs a)
     unsigned char *sA = smem_raw + kBBytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + kBBytes + kStages * kAStage);
     uint64_t *afull = bars, *aempty = bars + kStages, *tfull = bars + 2 * kStages, *tempty = tfull + 2;
-    uint64_t *bfull = tempty + 2, *bdone = bfull + 1, *drain = bdone + 1;
+    uint64_t *bfull = tempty + 2, *bdone = bfull + 1, *drain = bdone + 1, *handoff = drain + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kNBars);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(&afull[s], kProdThreads);
+            mbar_init(&afull[s], kProdGroupThreads);
             mbar_init(&aempty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
             mbar_init(&tempty[b], 32 * kEpiWarps);
+            mbar_init(&handoff[b], kProdGroupThreads);
         }
         mbar_init(bfull, 1);
         mbar_init(bdone, 1);
@@ -461,19 +492,27 @@ __global__ void __launch_bounds__(umma::kWsThreads, 1) k_dft_tcgen05(WsArgs a)
     const int u0 = (int)((long long)a.nunits * blockIdx.x / gridDim.x);
     const int u1 = (int)((long long)a.nunits * (blockIdx.x + 1) / gridDim.x);
     const long long lim = a.wait_cycles;
-    const int nparts = a.nnc * a.nkr;
 
     if (warp == kMmaWarp) {
         if (lane == 0) {
             // ---------------------------------------------------------------- MMA issue
+            // One thread issues 12 MMAs per chunk, so its own instructions count:
+            // the descriptors are a constant high word and a low word per stage or
+            // chunk plus immediate offsets (in 16-byte units), and the unit after
+            // this one is loaded ahead.
+            const uint32_t dhi = (uint32_t)(sdesc(0) >> 32), dlo = (uint32_t)sdesc(0);
+            const uint32_t a0 = dlo + (saddr(sA) >> 4), b0 = dlo + (saddr(sB) >> 4);
+            auto desc = [dhi](uint32_t lo) { return (uint64_t)dhi << 32 | lo; };
+            constexpr uint32_t kA = kABytes / 16, kB = kBArr * 2 / 16;  // one array of a stage, of a B chunk
             int cur_blk = -1;
-            uint32_t g = 0, nbf = 0, nbd = 0;  // A chunks consumed; bfull / bdone phases seen
-            bool b_pending = false;             // a block copy issued but not seen complete
+            uint32_t s = 0, ph = 0, nbf = 0, nbd = 0;  // A stage and its phase; bfull / bdone phases seen
+            bool b_pending = false;                     // a block copy issued but not seen complete
+            WsUnit next = a.units[u0];
             for (int i = u0; i < u1; ++i) {
-                const WsUnit un = a.units[i];
-                const int part = un.blk % nparts, nc = part / a.nkr, kr = part % a.nkr;
-                const int Nc = min(kN, a.D2p - kN * nc);
-                const int nkc = min(kKCB, (a.D1p - kKR * kr) / kKC);
+                const WsUnit un = next;
+                if (i + 1 < u1) next = a.units[i + 1];
+                const int Nc = min(kN, a.D2p - kN * (un.ncr & 0xFFFF));
+                const int nkc = min(kKCB, a.Kp / kKC - kKCB * (un.ncr >> 16));
                 bool ok = true;
                 if (un.blk != cur_blk) {
                     if (cur_blk >= 0) {  // the MMAs that read the resident block must be complete
@@ -495,31 +534,29 @@ __global__ void __launch_bounds__(umma::kWsThreads, 1) k_dft_tcgen05(WsArgs a)
                 tc_fence_after();
                 const uint32_t idesc = F16 ? idesc_f16(kM, Nc) : idesc_bf16(kM, Nc);
                 const uint32_t dre = tmem + (uint32_t)(buf * 256), dim = dre + 128;
-                for (int kc = 0; kc < nkc; ++kc, ++g) {
-                    const int s = (int)(g % kStages);
-                    if (!ws_wait(&afull[s], (g / kStages) & 1, lim, abort_flag)) {
+                for (int kc = 0; kc < nkc; ++kc) {
+                    if (!ws_wait(&afull[s], ph, lim, abort_flag)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    // the B chunk of this A chunk (pairs (p, H + p) in the mirrored order)
-                    const int bc = a.mirror ? ((kc & 1) ? a.mirror + (kc >> 1) : (kc >> 1)) : kc;
-                    const uint32_t a_base = saddr(sA + s * kAStage), b_base = saddr(sB + bc * kBChunk);
+                    const uint32_t al = a0 + s * (kAStage / 16), bl = b0 + (uint32_t)kc * (kBChunk / 16);
 #pragma unroll
                     for (int ks = 0; ks < 2; ++ks) {
-                        const uint32_t ko = ks * 16 * 16;  // 16 k = two core matrices = 256 bytes
-                        const uint64_t b_hi = sdesc(b_base + ko), b_lo = sdesc(b_base + kBArr * 2 + ko);
-                        const uint64_t a_rh = sdesc(a_base + ko), a_rl = sdesc(a_base + kABytes + ko);
-                        const uint64_t a_ih = sdesc(a_base + 2 * kABytes + ko), a_il = sdesc(a_base + 3 * kABytes + ko);
+                        const uint32_t x = al + ks * 16, y = bl + ks * 16;  // 16 k = two core matrices = 256 bytes
                         const uint32_t first = (kc == 0 && ks == 0) ? 0u : 1u;
-                        mma_bf16(dre, a_rh, b_hi, idesc, first);
-                        mma_bf16(dre, a_rh, b_lo, idesc, 1u);
-                        mma_bf16(dre, a_rl, b_hi, idesc, 1u);
-                        mma_bf16(dim, a_ih, b_hi, idesc, first);
-                        mma_bf16(dim, a_ih, b_lo, idesc, 1u);
-                        mma_bf16(dim, a_il, b_hi, idesc, 1u);
+                        mma_bf16(dre, desc(x), desc(y), idesc, first);
+                        mma_bf16(dre, desc(x), desc(y + kB), idesc, 1u);
+                        mma_bf16(dre, desc(x + kA), desc(y), idesc, 1u);
+                        mma_bf16(dim, desc(x + 2 * kA), desc(y + 2 * kB), idesc, first);
+                        mma_bf16(dim, desc(x + 2 * kA), desc(y + 3 * kB), idesc, 1u);
+                        mma_bf16(dim, desc(x + 3 * kA), desc(y + 2 * kB), idesc, 1u);
                     }
                     mma_commit(&aempty[s]);  // the stage is free once these MMAs have read it
+                    if (++s == kStages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
                 }
                 if (!ok) break;
                 mma_commit(&tfull[buf]);  // the unit's accumulator is complete
@@ -531,185 +568,176 @@ __global__ void __launch_bounds__(umma::kWsThreads, 1) k_dft_tcgen05(WsArgs a)
         }
     } else if (warp >= kProdWarp0) {
         // -------------------------------------------------------------------- A producers
-        const int q = tid - kProdWarp0 * 32;
-        const int r = q & (kM - 1), h = q >> 7;  // point (row) and half of the 32-wide chunk
+        const int pg = (warp - kProdWarp0) / kProdGroupWarps;      // units u0 + pg, u0 + pg + 2, ...
+        const int r = (tid - kProdWarp0 * 32) % kProdGroupThreads;  // point (row)
         const double inv1 = 1.0 / (double)a.n1;
-        const int amin = -(a.D1 / 2);
-        uint32_t g = 0;
-        bool ok = true;
-        for (int i = u0; i < u1 && ok; ++i) {
+        uint32_t g = 0;  // chunks before the unit
+        for (int i = u0; i < u1; ++i) {
             const WsUnit un = a.units[i];
-            const int kr = (un.blk % nparts) % a.nkr;
-            const int nkc = min(kKCB, (a.D1p - kKR * kr) / kKC);
+            const int kr = un.ncr >> 16;
+            const int nkc = min(kKCB, a.Kp / kKC - kKCB * kr);
+            if (((i - u0) & 1) != pg) {
+                g += nkc;
+                continue;
+            }
             const bool row_ok = r < un.nj;
             const float uj = row_ok ? a.u[un.j0 + r] : 0.f;
-            // rotations of the row: by 1 (odd elements), 2 (chain step), 4, 8, 12 (chain
-            // starts) and 32 (next chunk); the packed ones as ((x, x), (y, y), (-y, -y))
+            // rotations of the row by 1, 2, 4, 8, 16 (second half of a chunk) and 32
+            // (next chunk); the packed ones as ((x, x), (y, y), (-y, -y))
             const float2 w1 = phase_any<POW2>(1, uj, a.log2n1, inv1);
             const float2 w4 = phase_any<POW2>(4, uj, a.log2n1, inv1);
-            const float2 w2 = cmulf(w1, w1), w8 = cmulf(w4, w4), w12 = cmulf(w8, w4);
-            const float2 w32 = cmulf(cmulf(w8, w8), cmulf(w8, w8));
+            const float2 w2 = cmulf(w1, w1), w8 = cmulf(w4, w4);
+            const float2 w16 = cmulf(w8, w8), w32 = cmulf(w16, w16);
             const f2x_t w2x = pk(w2.x, w2.x), w2y = pk(w2.y, w2.y), w2n = pk(-w2.y, -w2.y);
             const f2x_t w4x = pk(w4.x, w4.x), w4y = pk(w4.y, w4.y), w4n = pk(-w4.y, -w4.y);
             const f2x_t w8x = pk(w8.x, w8.x), w8y = pk(w8.y, w8.y), w8n = pk(-w8.y, -w8.y);
-            const f2x_t wcx = pk(w12.x, w12.x), wcy = pk(w12.y, w12.y), wcn = pk(-w12.y, -w12.y);
+            // 8 consecutive k of row r from the pair (X0, Y0) of the first two (real
+            // parts packed, imaginary parts packed): pair 2 rotated from it by 4, pairs
+            // 1 and 3 from pairs 0 and 2 by 2; split into hi/lo words and stored at the
+            // row's 16 bytes of each array
+            auto eight = [&](f2x_t X0, f2x_t Y0, uint16_t *dst) {
+                f2x_t X[4], Y[4];
+                X[0] = X0; Y[0] = Y0;
+                X[2] = X0; Y[2] = Y0; rot_x2(X[2], Y[2], w4x, w4y, w4n);
+                X[1] = X0; Y[1] = Y0; rot_x2(X[1], Y[1], w2x, w2y, w2n);
+                X[3] = X[2]; Y[3] = Y[2]; rot_x2(X[3], Y[3], w2x, w2y, w2n);
+                uint32_t xh[4], xl[4], yh[4], yl[4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    split_x2<F16>(X[m], xh[m], xl[m]);
+                    split_x2<F16>(Y[m], yh[m], yl[m]);
+                }
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(xh[0], xh[1], xh[2], xh[3]);
+                *reinterpret_cast<uint4 *>(dst + kABytes / 2) = make_uint4(xl[0], xl[1], xl[2], xl[3]);
+                *reinterpret_cast<uint4 *>(dst + 2 * (kABytes / 2)) = make_uint4(yh[0], yh[1], yh[2], yh[3]);
+                *reinterpret_cast<uint4 *>(dst + 3 * (kABytes / 2)) = make_uint4(yl[0], yl[1], yl[2], yl[3]);
+            };
             float2 anchor = make_float2(0.f, 0.f);
-            // 16 consecutive k of row r from an anchor E_u(a): 8 pairs (2p, 2p+1), each
-            // pair's real parts and imaginary parts packed: pair 0 from the anchor,
-            // pairs 2, 4, 6 rotated from it by 4, 8, 12 and every odd pair from the one
-            // before it by 2 (four independent chains of packed rotations, at most
-            // three rotations from the anchor), split into hi/lo words
-            uint32_t rh[9], rl[9], ih[9], il[9];
-            auto gen = [&](float2 anc) {
-                const float2 e1 = cmulf(anc, w1);
-                f2x_t X[8], Y[8];
-                X[0] = pk(anc.x, e1.x);
-                Y[0] = pk(anc.y, e1.y);
-                X[2] = X[0]; Y[2] = Y[0]; rot_x2(X[2], Y[2], w4x, w4y, w4n);
-                X[4] = X[0]; Y[4] = Y[0]; rot_x2(X[4], Y[4], w8x, w8y, w8n);
-                X[6] = X[0]; Y[6] = Y[0]; rot_x2(X[6], Y[6], wcx, wcy, wcn);
-#pragma unroll
-                for (int m = 0; m < 8; m += 2) {
-                    X[m + 1] = X[m];
-                    Y[m + 1] = Y[m];
-                    rot_x2(X[m + 1], Y[m + 1], w2x, w2y, w2n);
+            bool ok = true;
+            for (int kc = 0; kc < nkc; ++kc, ++g) {
+                // 32 consecutive k of row r: a = 1 + 128 kr + 32 kc + 0..31; the anchor
+                // E_u(a) is exact at the block's first chunk and one rotation by 32
+                // from the previous chunk's otherwise
+                if (kc == 0)
+                    anchor = row_ok ? phase_any<POW2>(1 + kKR * kr, uj, a.log2n1, inv1) : make_float2(0.f, 0.f);
+                else
+                    anchor = cmulf(anchor, w32);
+                const float2 e1 = cmulf(anchor, w1);
+                f2x_t X = pk(anchor.x, e1.x), Y = pk(anchor.y, e1.y);
+                const float2 anchor2 = cmulf(anchor, w16), e2 = cmulf(anchor2, w1);
+                f2x_t X2 = pk(anchor2.x, e2.x), Y2 = pk(anchor2.y, e2.y);
+                // a unit's stages follow the other group's: its last unit's waits are
+                // done before this group waits for the same stages' next phases (a
+                // phase is told from the one before the last by nothing)
+                if (kc == 0 && i > u0 && !ws_wait(&handoff[1 - pg], ((i - u0 - 1) >> 1) & 1, lim, abort_flag)) {
+                    ok = false;
+                    break;
                 }
-#pragma unroll
-                for (int m = 0; m < 8; ++m) {
-                    split_x2<F16>(X[m], rh[m], rl[m]);
-                    split_x2<F16>(Y[m], ih[m], il[m]);
+                // the next A stage, once the MMAs that read it last have completed
+                const int st = (int)(g % kStages);
+                if (g >= (uint32_t)kStages && !ws_wait(&aempty[st], ((g / kStages) - 1) & 1, lim, abort_flag)) {
+                    ok = false;
+                    break;
                 }
-                // the 17th value, E_u(a + 16) = E_u(a + 15) E_u(1), in the low halves
-                const float2 v15 = make_float2(upk(X[7]).y, upk(Y[7]).y);
-                const float2 v16 = cmulf(v15, w1);
-                split_x2<F16>(pk(v16.x, 0.f), rh[8], rl[8]);
-                split_x2<F16>(pk(v16.y, 0.f), ih[8], il[8]);
-            };
-            // the next A stage, once the MMAs that read it last have completed
-            auto acquire = [&](int &st) -> bool {
-                st = (int)(g % kStages);
-                return g < (uint32_t)kStages || ws_wait(&aempty[st], ((g / kStages) - 1) & 1, lim, abort_flag);
-            };
-            auto store = [&](int st, const uint32_t *wrh, const uint32_t *wrl, const uint32_t *wih, const uint32_t *wil) {
-                uint16_t *As = reinterpret_cast<uint16_t *>(sA + st * kAStage);
-#pragma unroll
-                for (int c8 = 0; c8 < 2; ++c8) {
-                    const int idx = kmaj_index(r, 16 * h + 8 * c8);  // one 16-byte core-matrix row
-                    const int k0 = 4 * c8;
-                    *reinterpret_cast<uint4 *>(As + 0 * (kABytes / 2) + idx) = make_uint4(wrh[k0], wrh[k0 + 1], wrh[k0 + 2], wrh[k0 + 3]);
-                    *reinterpret_cast<uint4 *>(As + 1 * (kABytes / 2) + idx) = make_uint4(wrl[k0], wrl[k0 + 1], wrl[k0 + 2], wrl[k0 + 3]);
-                    *reinterpret_cast<uint4 *>(As + 2 * (kABytes / 2) + idx) = make_uint4(wih[k0], wih[k0 + 1], wih[k0 + 2], wih[k0 + 3]);
-                    *reinterpret_cast<uint4 *>(As + 3 * (kABytes / 2) + idx) = make_uint4(wil[k0], wil[k0 + 1], wil[k0 + 2], wil[k0 + 3]);
-                }
+                uint16_t *dst = reinterpret_cast<uint16_t *>(sA + st * kAStage) + kmaj_index(r, 0);
+                eight(X, Y, dst);
+                rot_x2(X, Y, w8x, w8y, w8n);
+                eight(X, Y, dst + 64);
+                eight(X2, Y2, dst + 128);
+                rot_x2(X2, Y2, w8x, w8y, w8n);
+                eight(X2, Y2, dst + 192);
                 fence_proxy_async();  // the stores are visible to the tensor core
                 mbar_arrive(&afull[st]);
-                ++g;
-            };
-            if (a.mirror) {
-                // K as a = 0 .. 32H-1, then a = -1 .. -32H: the chunk pair (p, H + p).
-                // The negative chunk's element k holds E_u(-(32p + k) - 1) =
-                // conj E_u(32p + k + 1): this thread's values shifted by one (its 17th
-                // value closes the row), the words re-paired by a byte permute and the
-                // imaginary parts negated by their sign bits (the hi/lo split of -x is
-                // -hi, -lo).  The anchor E_u(32p + 16h) is exact every 4 pairs.
-                for (int pp = 0; pp < nkc / 2; ++pp) {
-                    if ((pp & 3) == 0)
-                        anchor = row_ok ? phase_any<POW2>(kKC * pp + 16 * h, uj, a.log2n1, inv1) : make_float2(0.f, 0.f);
-                    else
-                        anchor = cmulf(anchor, w32);
-                    gen(anchor);
-                    int st;
-                    if (!acquire(st)) { ok = false; break; }
-                    store(st, rh, rl, ih, il);
-                    uint32_t nrh[8], nrl[8], nih[8], nil[8];
-#pragma unroll
-                    for (int m = 0; m < 8; ++m) {
-                        nrh[m] = __byte_perm(rh[m], rh[m + 1], 0x5432);
-                        nrl[m] = __byte_perm(rl[m], rl[m + 1], 0x5432);
-                        nih[m] = __byte_perm(ih[m], ih[m + 1], 0x5432) ^ 0x80008000u;
-                        nil[m] = __byte_perm(il[m], il[m + 1], 0x5432) ^ 0x80008000u;
-                    }
-                    if (!acquire(st)) { ok = false; break; }
-                    store(st, nrh, nrl, nih, nil);
-                }
-            } else {
-                for (int kc = 0; kc < nkc; ++kc) {
-                    // 16 consecutive k of row r: a = amin + kr*256 + kc*32 + 16h + 0..15; the
-                    // anchor E_u(a) is exact every 4 chunks and one rotation by 32 from the
-                    // previous chunk's otherwise
-                    if ((kc & 3) == 0)
-                        anchor = row_ok ? phase_any<POW2>(amin + kKR * kr + kKC * kc + 16 * h, uj, a.log2n1, inv1)
-                                        : make_float2(0.f, 0.f);
-                    else
-                        anchor = cmulf(anchor, w32);
-                    gen(anchor);
-                    int st;
-                    if (!acquire(st)) { ok = false; break; }
-                    store(st, rh, rl, ih, il);
-                }
             }
+            if (!ok) break;
+            mbar_arrive(&handoff[pg]);
         }
     } else {
         // -------------------------------------------------------------------- epilogue
-        const int row = warp * 32 + lane;  // TMEM lane of this warp's quadrant
+        const int grp = warp / kEpiWarps;                // units u0 + grp, u0 + grp + 2, ...: accumulator buffer grp
+        const int row = (warp % kEpiWarps) * 32 + lane;  // TMEM lane of this warp's quadrant
         const double inv2 = 1.0 / (double)a.n2;
         const int bmin = -(a.D2 / 2);
-        const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-        for (int i = u0; i < u1; ++i) {
-            const WsUnit un = a.units[i];
-            const int part = un.blk % nparts, nc = part / a.nkr;
+        const uint32_t lane_base = (uint32_t)((warp % kEpiWarps) * 32) << 16;
+        // the next unit and its point's v are loaded while the current one is
+        // contracted, and the phases are formed before the wait for its accumulators
+        WsUnit un = a.units[min(u0 + grp, u1 - 1)];
+        float vj = row < un.nj ? a.v[un.j0 + row] : 0.f;
+        for (int i = u0 + grp; i < u1; i += 2) {
+            const int nc = un.ncr & 0xFFFF, kr = un.ncr >> 16, part = nc * a.nkr + kr;
             const int Nc = min(kN, a.D2p - kN * nc);
+            const float4 *p0 = reinterpret_cast<const float4 *>(a.P0 + (size_t)un.proj * a.D2p + kN * nc);
             const int li = i - u0, buf = li & 1;
-            if (!ws_wait(&tfull[buf], (li >> 1) & 1, lim, abort_flag)) break;
-            tc_fence_after();
             const bool row_ok = row < un.nj;
-            const float vj = row_ok ? a.v[un.j0 + row] : 0.f;
             const float2 v1 = phase_any<POW2>(1, vj, a.log2n2, inv2);
             const float2 v16 = phase_any<POW2>(16, vj, a.log2n2, inv2);
-            const float2 v2 = cmulf(v1, v1);
+            float2 an = row_ok ? phase_any<POW2>(bmin + kN * nc, vj, a.log2n2, inv2) : make_float2(0.f, 0.f);
+            const float2 an64 = row_ok ? phase_any<POW2>(bmin + kN * nc + 64, vj, a.log2n2, inv2) : make_float2(0.f, 0.f);
+            const float2 v2 = cmulf(v1, v1), v4 = cmulf(v2, v2), v8 = cmulf(v4, v4);
             const f2x_t v2x = pk(v2.x, v2.x), v2y = pk(v2.y, v2.y), v2n = pk(-v2.y, -v2.y);
+            WsUnit next = un;
+            float vnext = 0.f;
+            if (i + 2 < u1) {
+                next = a.units[i + 2];
+                if (row < next.nj) vnext = a.v[next.j0 + row];
+            }
+            if (!ws_wait(&tfull[buf], (li >> 1) & 1, lim, abort_flag)) break;
+            tc_fence_after();
             const uint32_t cre = tmem + lane_base + (uint32_t)(buf * 256), cim = cre + 128;
-            float2 Fsum = make_float2(0.f, 0.f), an = make_float2(0.f, 0.f);
-            // F += sum_b Q(j,b) E_v(j,b) over 16-column groups: with w = E_v(1), a group's
-            // sum_i Q_i w^i is A(w^2) + w B(w^2), A and B the polynomials of its even and
-            // odd columns, both evaluated by Horner's rule in one packed chain (the pair
-            // (A, B) of real parts and the pair of imaginary parts), then multiplied by
-            // the group's anchor E_v(b_g) (exact every 64 columns, one rotation by 16
-            // from the previous group otherwise); two groups per step (independent
-            // chains, one wait for both loads)
-            auto group = [&](const uint32_t(&re)[16], const uint32_t(&im)[16], float2 anc) {
-                f2x_t H = pk(__uint_as_float(re[14]), __uint_as_float(re[15]));
-                f2x_t G = pk(__uint_as_float(im[14]), __uint_as_float(im[15]));
-#pragma unroll
-                for (int t = 6; t >= 0; --t) {
-                    const f2x_t qr = pk(__uint_as_float(re[2 * t]), __uint_as_float(re[2 * t + 1]));
-                    const f2x_t qi = pk(__uint_as_float(im[2 * t]), __uint_as_float(im[2 * t + 1]));
-                    const f2x_t h2 = fma_x2(H, v2x, fma_x2(G, v2n, qr));
+            float2 Fsum = make_float2(0.f, 0.f);
+            // F += sum_b Q(j,b) E_v(j,b), eight columns at a time: with w = E_v(1),
+            // sum_i Q_i w^i is A(w^2) + w B(w^2), A and B the polynomials of the even
+            // and odd columns, both evaluated by Horner's rule in one packed chain (the
+            // pair (A, B) of real parts and the pair of imaginary parts).  Sixteen
+            // columns are two such sums, joined by w^8 and multiplied by their anchor
+            // E_v(b_g) (exact every 64 columns, one rotation by 16 from the previous
+            // one otherwise).  The next eight columns are loaded while these are
+            // contracted.  The real part's row a = 0, the same for all points, joins
+            // here: its columns' pairs are broadcast loads, in the first K block's units.
+            struct Eight {
+                uint32_t re[8], im[8];
+                float4 z0, z1;
+            };
+            auto load = [&](Eight &e, int c) {
+                tmem_ld8(cre + (uint32_t)c, e.re);
+                tmem_ld8(cim + (uint32_t)c, e.im);
+                e.z0 = e.z1 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (kr == 0) {
+                    e.z0 = __ldg(p0 + c / 4);
+                    e.z1 = __ldg(p0 + c / 4 + 1);
+                }
+            };
+            auto eight = [&](const Eight &e) -> float2 {
+                auto re = [&](int t) { return pk(__uint_as_float(e.re[2 * t]), __uint_as_float(e.re[2 * t + 1])); };
+                auto im = [&](int t) { return pk(__uint_as_float(e.im[2 * t]), __uint_as_float(e.im[2 * t + 1])); };
+                const f2x_t q0 = add_x2(re(0), pk(e.z0.x, e.z0.y)), q1 = add_x2(re(1), pk(e.z0.z, e.z0.w));
+                const f2x_t q2 = add_x2(re(2), pk(e.z1.x, e.z1.y)), q3 = add_x2(re(3), pk(e.z1.z, e.z1.w));
+                f2x_t H = q3, G = im(3);
+                auto step = [&](f2x_t q, f2x_t qi) {
+                    const f2x_t h2 = fma_x2(H, v2x, fma_x2(G, v2n, q));
                     G = fma_x2(H, v2y, fma_x2(G, v2x, qi));
                     H = h2;
-                }
+                };
+                step(q2, im(2));
+                step(q1, im(1));
+                step(q0, im(0));
                 const float2 hr = upk(H), hi = upk(G);  // (A.re, B.re), (A.im, B.im)
                 const float2 sB = cmulf(make_float2(hr.y, hi.y), v1);
-                const float2 p = cmulf(make_float2(hr.x + sB.x, hi.x + sB.y), anc);
+                return make_float2(hr.x + sB.x, hi.x + sB.y);
+            };
+            Eight e0, e1;
+            load(e0, 0);
+            for (int c = 0; c < Nc; c += 16) {  // (Nc is a multiple of 16)
+                tmem_wait_ld();
+                load(e1, c + 8);
+                const float2 lo = eight(e0);
+                tmem_wait_ld();
+                if (c + 16 < Nc) load(e0, c + 16);
+                const float2 up = cmulf(eight(e1), v8);
+                const float2 p = cmulf(make_float2(lo.x + up.x, lo.y + up.y), an);
                 Fsum.x += p.x;
                 Fsum.y += p.y;
-            };
-            for (int c = 0; c < Nc; c += 32) {
-                const bool two = c + 16 < Nc;  // warp-uniform
-                uint32_t re0[16], im0[16], re1[16], im1[16];
-                tmem_ld16(cre + (uint32_t)c, re0);
-                tmem_ld16(cim + (uint32_t)c, im0);
-                if (two) {
-                    tmem_ld16(cre + (uint32_t)(c + 16), re1);
-                    tmem_ld16(cim + (uint32_t)(c + 16), im1);
-                }
-                const float2 an0 = (c & 63) == 0 ? (row_ok ? phase_any<POW2>(bmin + kN * nc + c, vj, a.log2n2, inv2)
-                                                          : make_float2(0.f, 0.f))
-                                                 : cmulf(an, v16);
-                an = cmulf(an0, v16);  // the second group's anchor
-                tmem_wait_ld();
-                group(re0, im0, an0);
-                if (two) group(re1, im1, an);
+                an = (c & 63) == 48 ? an64 : cmulf(an, v16);  // the next sixteen's
             }
             tc_fence_before();
             mbar_arrive(&tempty[buf]);  // this thread's TMEM reads of the buffer are complete
@@ -717,6 +745,8 @@ __global__ void __launch_bounds__(umma::kWsThreads, 1) k_dft_tcgen05(WsArgs a)
                 const float sc = a.inv_scale[un.proj];
                 a.F[(size_t)part * a.ntot + un.j0 + row] = make_float2(Fsum.x * sc, Fsum.y * sc);
             }
+            un = next;
+            vj = vnext;
         }
     }
 
@@ -766,6 +796,7 @@ constexpr int kWNBars = 2 * kWStages + 4 + 3;         // afull, aempty, tfull x2
 // roles: warps 0-7 epilogue (warp w drains accumulator buffer w / 4, quadrant
 // w % 4), warp 8 MMA issue and block copies, warps 9-16 A producers
 constexpr int kWMmaWarp = 8, kWProdWarp0 = 9;  // warps 0 .. kWMmaWarp - 1 are the epilogue
+constexpr int kProdWarps = 8, kProdThreads = 32 * kProdWarps;
 constexpr int kWThreads = 32 * (kWProdWarp0 + kProdWarps);  // 544
 constexpr size_t kWSmem = (size_t)kWBBytes + (size_t)kWStages * kWAStage + 8 * kWNBars + 16;
 static_assert(kWSmem <= 227 * 1024, "shared memory of the N = 256 form");
@@ -831,7 +862,7 @@ __global__ void __launch_bounds__(umma::kWThreads, 1) k_dft_tcgen05_w(WsArgs a)
                 const WsUnit un = a.units[i];
                 const int part = un.blk % nparts, nc = part / a.nkr, kr = part % a.nkr;
                 const int Nc = min(kWN, a.D2p - kWN * nc);
-                const int nkc = min(kWKCB, (a.D1p - kWKR * kr) / kKC);
+                const int nkc = min(kWKCB, (a.Kp - kWKR * kr) / kKC);
                 bool ok = true;
                 if (un.blk != cur_blk) {
                     if (cur_blk >= 0) {
@@ -892,7 +923,7 @@ __global__ void __launch_bounds__(umma::kWThreads, 1) k_dft_tcgen05_w(WsArgs a)
         for (int i = u0; i < u1 && ok; ++i) {
             const WsUnit un = a.units[i];
             const int kr = (un.blk % nparts) % a.nkr;
-            const int nkc = min(kWKCB, (a.D1p - kWKR * kr) / kKC);
+            const int nkc = min(kWKCB, (a.Kp - kWKR * kr) / kKC);
             const bool row_ok = pt < un.nj;
             const float uj = row_ok ? a.u[un.j0 + pt] : 0.f;
             const float2 w1 = phase_any<POW2>(1, uj, a.log2n1, inv1);
@@ -1048,43 +1079,72 @@ __global__ void __launch_bounds__(256) k_proj_scale(const double *__restrict__ p
     }
 }
 
-// Pre-split (scaled) projections into hi/lo blocks in the B layout: block
-// (p, nc, kr) holds columns b = NB nc + (0..NB-1) and rows a = KR kr + (0..KR-1)
-// as KR / 32 K chunks of [hi | lo][NB x 32]; zero beyond D1 x D2.  NB x KR is
-// 128 x 256 (first form) or 256 x 128 (second form), 128 KB either way.
+// hi and lo of x in the 16-bit operand type, at dst[0] and dst[stride]
+template <bool F16> __device__ __forceinline__ void split_to(float x, uint16_t *dst, int stride)
+{
+    if constexpr (F16) {
+        const __half hi = __float2half_rn(x);
+        dst[0] = __half_as_ushort(hi);
+        dst[stride] = __half_as_ushort(__float2half_rn(x - __half2float(hi)));
+    } else {
+        const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+        dst[0] = __bfloat16_as_ushort(hi);
+        dst[stride] = __bfloat16_as_ushort(__float2bfloat16_rn(x - __bfloat162float(hi)));
+    }
+}
+
+// First form's B blocks: folded (scaled) projections, split into hi and lo.
+// Block (p, nc, kr) holds columns b = 128 nc + 0..127 and folded rows
+// a = 1 + 128 kr + 0..127 as 4 K chunks of [Pe hi | Pe lo | Po hi | Po lo][128 x 32];
+// zero beyond the projection.  P0 (D2p per projection) receives row a = 0.
 // Grid: x = block, y = K chunk.
-template <bool F16, int NB, int KR>
+template <bool F16>
+__global__ void __launch_bounds__(256) k_fold_split(const double *__restrict__ proj, int D1, int D2, int D2p, int nnc,
+                                                    int nkr, const float *__restrict__ scale, uint16_t *__restrict__ B,
+                                                    float *__restrict__ P0)
+{
+    using namespace umma;
+    const int blk = blockIdx.x, kc = blockIdx.y;
+    const int kr = blk % nkr, nc = (blk / nkr) % nnc, p = blk / (nkr * nnc);
+    const double *src = proj + (long long)p * D1 * D2;
+    const double sc = (double)scale[p];
+    const int m = D1 / 2;
+    uint16_t *dst = B + (size_t)blk * (kBBytes / 2) + (size_t)kc * (kBChunk / 2);
+    for (int e = threadIdx.x; e < kBArr; e += 256) {
+        // e is the linear position in the layout: invert kmaj_index
+        const int rg = e >> 8, kg = (e >> 6) & 3, rr = (e >> 3) & 7, kk = e & 7;
+        const int a = 1 + kr * kKR + kc * kKC + kg * 8 + kk, b = nc * kN + rg * 8 + rr;
+        double x = 0.0, y = 0.0;  // P(a, b) and P(-a, b)
+        if (b < D2 && a <= m) {
+            if (m + a < D1) x = src[m + a + (long long)D1 * b];
+            y = src[m - a + (long long)D1 * b];
+        }
+        split_to<F16>((float)((x + y) * sc), dst + e, kBArr);
+        split_to<F16>((float)((x - y) * sc), dst + 2 * kBArr + e, kBArr);
+    }
+    if (kr == 0 && kc == 0)
+        for (int b = nc * kN + threadIdx.x; b < min(D2p, (nc + 1) * kN); b += 256)
+            P0[(size_t)p * D2p + b] = b < D2 ? (float)(src[m + (long long)D1 * b] * sc) : 0.f;
+}
+
+// Second form's B blocks: block (p, nc, kr) holds columns b = 256 nc + 0..255
+// and rows a = 128 kr + 0..127 (from the projection's first) as 4 K chunks of
+// [hi | lo][256 x 32]; zero beyond D1 x D2.  Grid: x = block, y = K chunk.
+template <bool F16>
 __global__ void __launch_bounds__(256) k_split_projections(const double *__restrict__ proj, int D1, int D2, int nnc,
-                                                           int nkr, int mirror_m, const float *__restrict__ scale,
+                                                           int nkr, const float *__restrict__ scale,
                                                            uint16_t *__restrict__ B)
 {
     using namespace umma;
-    constexpr int kArr = NB * kKC;                 // elements of one array of a chunk
-    constexpr int kBlk = (KR / kKC) * 2 * kArr;    // elements of one block
     const int blk = blockIdx.x, kc = blockIdx.y;
     const int kr = blk % nkr, nc = (blk / nkr) % nnc, p = blk / (nkr * nnc);
     const double *src = proj + (long long)p * D1 * D2;
     const float sc = scale[p];
-    uint16_t *dst = B + (size_t)blk * kBlk + (size_t)kc * (2 * kArr);
-    for (int e = threadIdx.x; e < kArr; e += 256) {
-        // e is the linear position in the layout: invert kmaj_index
+    uint16_t *dst = B + (size_t)blk * (kWBBytes / 2) + (size_t)kc * (kWBChunk / 2);
+    for (int e = threadIdx.x; e < kWBArr; e += 256) {
         const int rg = e >> 8, kg = (e >> 6) & 3, rr = (e >> 3) & 7, kk = e & 7;
-        // K row: natural (aa = a + D1/2), or with mirror_m = D1/2 the order
-        // a = 0 .. m-1 then a = -1 .. -m (see WsArgs::mirror)
-        const int kabs = kc * kKC + kg * 8 + kk;
-        const int b = nc * NB + rg * 8 + rr;
-        const int aa = mirror_m ? (kabs < mirror_m ? kabs + mirror_m : 2 * mirror_m - 1 - kabs) : kr * KR + kabs;
-        // rows outside 0 .. D1-1 (the block's padding, in either order) are zero
-        const float xf = (b < D2 && aa >= 0 && aa < D1) ? (float)src[aa + (long long)D1 * b] * sc : 0.f;
-        if constexpr (F16) {
-            const __half hi = __float2half_rn(xf);
-            dst[e] = __half_as_ushort(hi);
-            dst[kArr + e] = __half_as_ushort(__float2half_rn(xf - __half2float(hi)));
-        } else {
-            const __nv_bfloat16 hi = __float2bfloat16_rn(xf);
-            dst[e] = __bfloat16_as_ushort(hi);
-            dst[kArr + e] = __bfloat16_as_ushort(__float2bfloat16_rn(xf - __bfloat162float(hi)));
-        }
+        const int aa = kr * kWKR + kc * kKC + kg * 8 + kk, b = nc * kWN + rg * 8 + rr;
+        split_to<F16>((b < D2 && aa < D1) ? (float)src[aa + (long long)D1 * b] * sc : 0.f, dst + e, kWBArr);
     }
 }
 
@@ -1155,7 +1215,8 @@ __global__ void __launch_bounds__(256) k_make_units(const long long *__restrict_
     const long long tiles = (nk + tp - 1) / tp, local = u - uoff[p];
     const long long t = local % tiles, rest = local / tiles;
     const int kr = (int)(rest % nkr), nc = (int)(rest / nkr);
-    units[u] = WsUnit{off[p] + t * tp, p, (p * nnc + nc) * nkr + kr, (int)min((long long)tp, nk - t * tp), 0};
+    units[u] = WsUnit{off[p] + t * tp, p, (p * nnc + nc) * nkr + kr, (int)min((long long)tp, nk - t * tp),
+                       nc | kr << 16};
 }
 
 __global__ void k_fill_f32(float *__restrict__ x, int n, float v)
@@ -1190,14 +1251,6 @@ static bool dft_use_wide()
     return e && std::strcmp(e, "n256") == 0;
 }
 
-// The first form's mirrored K order (WsArgs::mirror) where the shape allows it;
-// GENFIRE_DFT_MIRROR=0 keeps the natural order.
-static bool dft_mirror_enabled()
-{
-    const char *e = std::getenv("GENFIRE_DFT_MIRROR");
-    return !(e && e[0] == '0');
-}
-
 // Host: F (float2, one per selected point) for all projections.  Everything is
 // enqueued on the context stream without a host synchronisation: the unit list
 // and the scales are made on the device, and the error flag is the caller's to
@@ -1210,8 +1263,9 @@ void dft_tcgen05(genfire_ctx *ctx, const double *d_proj, int D1, int D2, int n1,
     cudaStream_t st = ctx->stream;
     const bool wide = dft_use_wide();
     const int NB = wide ? kWN : kN, KR = wide ? kWKR : kKR;  // block shape
-    const int D1p = (D1 + kKC - 1) / kKC * kKC, D2p = (D2 + 15) / 16 * 16;
-    const int nnc = (D2p + NB - 1) / NB, nkr = (D1p + KR - 1) / KR;
+    const int K = wide ? D1 : D1 / 2;  // the first form's rows are folded
+    const int Kp = (K + kKC - 1) / kKC * kKC, D2p = (D2 + 15) / 16 * 16;
+    const int nnc = (D2p + NB - 1) / NB, nkr = (Kp + KR - 1) / KR;
     const int nparts = nnc * nkr;
     const int nblk = P * nnc * nkr;
     const int tp = wide ? kWPoints : kM;  // points per tile
@@ -1224,7 +1278,7 @@ void dft_tcgen05(genfire_ctx *ctx, const double *d_proj, int D1, int D2, int n1,
     if (nunits > INT32_MAX) fail(GENFIRE_ERR_ARG, "tensor-core gridding: too many selected points.");
 
     static_assert(kBBytes == kWBBytes, "both block shapes hold 128 KB");
-    DevBuf B((size_t)nblk * kBBytes, st), scl(2 * sizeof(float) * P, st);
+    DevBuf B((size_t)nblk * kBBytes, st), scl(2 * sizeof(float) * P, st), P0;
     float *d_scale = scl.as<float>(), *d_inv = d_scale + P;
     if (fp16) {
         k_proj_scale<<<P, 256, 0, st>>>(d_proj, (long long)D1 * D2, d_scale, d_inv);
@@ -1232,17 +1286,15 @@ void dft_tcgen05(genfire_ctx *ctx, const double *d_proj, int D1, int D2, int n1,
         k_fill_f32<<<(2 * P + 255) / 256, 256, 0, st>>>(d_scale, 2 * P, 1.f);
     }
     GF_CHECK_LAUNCH();
-    // the mirrored K order of the first form: one K block of D1 = 64 H rows
-    const int mirror = (!wide && D1 % 64 == 0 && D1 <= kKR && dft_mirror_enabled()) ? D1 / 64 : 0;
     const dim3 sgrid((unsigned)nblk, KR / kKC);
     uint16_t *dB = B.as<uint16_t>();
     if (wide) {
-        if (fp16) k_split_projections<true, kWN, kWKR><<<sgrid, 256, 0, st>>>(d_proj, D1, D2, nnc, nkr, 0, d_scale, dB);
-        else k_split_projections<false, kWN, kWKR><<<sgrid, 256, 0, st>>>(d_proj, D1, D2, nnc, nkr, 0, d_scale, dB);
+        if (fp16) k_split_projections<true><<<sgrid, 256, 0, st>>>(d_proj, D1, D2, nnc, nkr, d_scale, dB);
+        else k_split_projections<false><<<sgrid, 256, 0, st>>>(d_proj, D1, D2, nnc, nkr, d_scale, dB);
     } else {
-        const int mm = mirror ? D1 / 2 : 0;
-        if (fp16) k_split_projections<true, kN, kKR><<<sgrid, 256, 0, st>>>(d_proj, D1, D2, nnc, nkr, mm, d_scale, dB);
-        else k_split_projections<false, kN, kKR><<<sgrid, 256, 0, st>>>(d_proj, D1, D2, nnc, nkr, mm, d_scale, dB);
+        P0.alloc(sizeof(float) * (size_t)P * D2p, st);
+        if (fp16) k_fold_split<true><<<sgrid, 256, 0, st>>>(d_proj, D1, D2, D2p, nnc, nkr, d_scale, dB, P0.as<float>());
+        else k_fold_split<false><<<sgrid, 256, 0, st>>>(d_proj, D1, D2, D2p, nnc, nkr, d_scale, dB, P0.as<float>());
     }
     GF_CHECK_LAUNCH();
 
@@ -1255,6 +1307,7 @@ void dft_tcgen05(genfire_ctx *ctx, const double *d_proj, int D1, int D2, int n1,
     DevBuf Fp(nparts > 1 ? sizeof(float2) * (size_t)nparts * ntot : 0, st);
     WsArgs a;
     a.B = B.as<uint16_t>();
+    a.P0 = P0.as<float>();
     a.units = du.as<WsUnit>();
     a.nunits = (int)nunits;
     a.u = d_u;
@@ -1262,12 +1315,11 @@ void dft_tcgen05(genfire_ctx *ctx, const double *d_proj, int D1, int D2, int n1,
     a.inv_scale = d_inv;
     a.F = nparts > 1 ? Fp.as<float2>() : d_F;
     a.ntot = ntot;
-    a.D1 = D1; a.D2 = D2; a.D1p = D1p; a.D2p = D2p;
+    a.D1 = D1; a.D2 = D2; a.Kp = Kp; a.D2p = D2p;
     a.n1 = n1; a.n2 = n2;
     auto lg = [](int n) { int t = 0; while ((1 << t) < n) ++t; return (1 << t) == n ? t : -1; };
     a.log2n1 = lg(n1); a.log2n2 = lg(n2);
     a.nnc = nnc; a.nkr = nkr;
-    a.mirror = mirror;
     a.err = d_err;
     // GENFIRE_DEBUG_DFT_WAIT_CYCLES (a positive count of clock cycles) shortens
     // the pipeline's waits so that a test can make one expire and exercise the
