@@ -466,6 +466,15 @@ static bool rows_r32_enabled()
     return !(e && e[0] == '1');
 }
 
+// the engine launch_rows takes for complex64 rows of n points, as a column variant
+static int row_engine(int n)
+{
+    if ((n == 512 || n == 1024) && rows_r32_enabled()) return kColR32;
+    if (two_fixed(n)) return kColTwo;
+    if (n == 64 || n == 128 || n == 256 || n == 512 || n == 1024) return kColReg1;
+    return mix_capable<float>(n) ? kColMix : two_capable<float>(n) ? kColTwo : kColGeneric;
+}
+
 template <typename T> static void launch_rows(RowPassArgs<T> a, bool forward, cudaStream_t st)
 {
     a.P = a.W + 1;
@@ -525,6 +534,66 @@ __global__ void __launch_bounds__(256) k_half_from_centered(const cplx<T> *__res
         const int a1 = q1 + c;  // q1 = n1 / 2 of an even n1 is the row's first entry, and its own mate
         const cplx<T> x = ra[a1 < n1 ? a1 : a1 - n1], y = rb[c - q1];
         row[q1] = mk((T)0.5 * (x.x + y.x), (T)0.5 * (x.y - y.y));
+    }
+}
+
+// Mean gain (squared length, less 1) of a complex64 transform of n points on a
+// column engine (variant), from the rounding of its twiddles and constants: a
+// rounded root has length 1 + a few 1e-8, the constants of a butterfly do not
+// average out, and a forward and inverse pair scales the object by 1 + the gain
+// (512 points on the radix-32 engine: -1e-7).  An iteration leaves the unmeasured
+// frequencies as they are, so over many of them this bias adds up where the
+// roundings' noise does not; the last pass of the inverse takes its mean back
+// (RowPassArgs::scale_lo).
+static double pass_gain(int variant, int n)
+{
+    auto twiddles_of = [](int ns, int R) {  // W_(ns R)^(k r), k < ns, r < R
+        double g = 0;
+        for (int k = 0; k < ns; ++k)
+            for (int r = 0; r < R; ++r) g += root_gain(k * r, ns * R);
+        return g / (ns * R);
+    };
+    auto stages = [&](const FftPlan &pl) {  // a Stockham schedule
+        double g = 0;
+        for (int st = 0, ns = 1; st < pl.nst; ns *= pl.radix(st), ++st)
+            g += (ns > 1 ? twiddles_of(ns, pl.radix(st)) : 0.0) + radix_gain(pl.radix(st));
+        return g;
+    };
+    FftPlan pl;
+    switch (variant) {
+    case kColTwo: return two_gain(n);
+    case kColMix: {
+        const int N1 = n % 3 == 0 ? 3 : 5, N2 = n / N1;
+        make_fft_plan(N2, pl);
+        return stages(pl) + twiddles_of(N2, N1) + radix_gain(N1);
+    }
+    case kColR32:
+    case kColR32Tma: {
+        // 32 points as 4 x 8, then 4, 8, 4 x 4 or 4 x 8; the twiddles between
+        // them by the products of r32_fft
+        double g = radix_gain(32);
+        const int P = n / 32;
+        g += P == 4 ? 0.0 : P == 8 ? radix_gain(8) : P == 16 ? radix_gain(16) : radix_gain(32);
+        auto root = [n](int j) {
+            return make_float2((float)root_cos(j % n, n), (float)-root_sin(j % n, n));
+        };
+        auto mul = [](float2 u, float2 v) {
+            return make_float2(std::fma(u.x, v.x, -(u.y * v.y)), std::fma(u.x, v.y, u.y * v.x));
+        };
+        double c = 0;
+        for (int t = 0; t < P; ++t)
+            for (int b = 0; b < 4; ++b) {
+                float2 w[8];
+                w[0] = root(t * b);
+                for (int a = 1; a < 8; ++a) {
+                    const int step = n >= 512 ? 1 : a >= 4 ? 4 : a >= 2 ? 2 : 1;
+                    w[a] = b == 0 && a == step ? root(4 * t * step) : mul(w[a - step], root(4 * t * step));
+                }
+                for (int a = 0; a < 8; ++a) c += (double)w[a].x * w[a].x + (double)w[a].y * w[a].y - 1.0;
+            }
+        return g + c / n;
+    }
+    default: make_fft_plan(n, pl); return stages(pl);
     }
 }
 
@@ -593,7 +662,7 @@ static void rec_ifft_t(genfire_ctx *ctx, const cplx<T> *d_M, int n1, int n2, int
     std::memset(&r, 0, sizeof(r));
     r.pl = c.pl1; r.tw = c.tw1; r.W = c.W1; r.nrows = D2 * D1; r.B1 = D1; r.c1 = D1 / 2; r.h1 = c.h1; r.ld1 = c.ld1;
     r.xs[0] = d_rec; r.xsel = nullptr; r.Y = Z.as<cplx<T>>();
-    inverse_scale<T>(r, (double)n1 * n2 * n1, 0.0);
+    inverse_scale<T>(r, (double)n1 * n2 * n1, 0.0);  // (one transform: the noise hides its mean gain)
     launch_rows<T>(r, false, st);
 }
 
@@ -1293,24 +1362,19 @@ template <typename T> struct ReconT : ReconBase {
         GF_CUDA(cudaStreamSynchronize(st));
     }
 
-    // the mean gain of the iteration's forward and inverse transforms, where they
-    // run on the two-stage engine (two_gain; the other engines' is left as it is)
-    double transform_gain() const
+    // the mean gain of the iteration's forward and inverse transforms: rows by
+    // launch_rows' engine, columns by launch_colpass'
+    double transform_gain()
     {
         if constexpr (sizeof(T) == 8) return 0.0;
-        auto column = [](ColPassArgs<T> a, int v) {  // the engine launch_colpass takes for a pass
+        auto column = [](const ColPassArgs<T> &a, int v) {
             const int f = forced_col_variant();
             if (f != kColAuto && col_variant_ok(a, f)) v = f;
             if (v == kColAuto || !col_variant_ok(a, v)) v = default_col_variant(a);
-            return v == kColTwo;
+            return pass_gain(v, a.pl.n);
         };
-        ReconT *self = const_cast<ReconT *>(this);
-        double g = 0;
-        if (two_fixed(n1)) g += two_gain(n1);
-        if (column(self->f2_args(), vF2)) g += 0.5 * two_gain(n2);
-        if (column(self->i2_args(false), vI2)) g += 0.5 * two_gain(n2);
-        if (column(self->f3_args(), vF3)) g += two_gain(n1);
-        return g;
+        return pass_gain(row_engine(n1), n1) + column(f3_args(), vF3) +
+               0.5 * (column(f2_args(), vF2) + column(i2_args(false), vI2));
     }
 
     // ev (optional) receives an event before each of the 7 kernels and one after

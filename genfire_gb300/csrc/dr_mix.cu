@@ -233,8 +233,8 @@ __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_row_c2r_mix(RowPas
             int e = k2 + N2 * k1 + a.c1;
             if (e >= N) e -= N;
             if (e < a.B1) {
-                if (r0 < a.nrows) x[(long long)r0 * a.B1 + e] = v[k1][k].x * a.scale;
-                if (r1 < a.nrows) x[(long long)r1 * a.B1 + e] = v[k1][k].y * a.scale;
+                if (r0 < a.nrows) x[(long long)r0 * a.B1 + e] = scaled(v[k1][k].x, a);
+                if (r1 < a.nrows) x[(long long)r1 * a.B1 + e] = scaled(v[k1][k].y, a);
             }
         }
     }

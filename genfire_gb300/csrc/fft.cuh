@@ -596,12 +596,18 @@ template <typename T> struct RowPassArgs {
     int positivity;
     cplx<T> *Y;        // ld1 x nrows half spectrum
     T scale;           // inverse only
-    T scale_lo;        // what scale misses of the exact factor (two-stage passes; 0 elsewhere)
+    T scale_lo;        // inverse, complex64: what scale misses of the exact factor
     // with ctl set (the iteration's first pass): CTA 0 starts the iteration
     // (ctl_begin_update) while every CTA reads the object from xs[ctl->xnext]
     Ctl *ctl;
     const int *changes;
 };
+
+// a value times an inverse row pass's factor: one more multiply-add in FP32
+// gives it 48 bits, so that neither the rounding of 1/N nor the transforms' mean
+// gain (see pass_gain in dr.cu) scales the object at every iteration
+__device__ __forceinline__ float scaled(float x, const RowPassArgs<float> &a) { return fmaf(x, a.scale, x * a.scale_lo); }
+__device__ __forceinline__ double scaled(double x, const RowPassArgs<double> &a) { return x * a.scale; }
 
 // The CTA's row pairs [blockIdx.x W, (blockIdx.x + 1) W) hold no support voxel
 // (RowPassArgs::pairmask); every thread reaches the same answer.  The W loads
@@ -704,8 +710,8 @@ __global__ void __launch_bounds__(kTileMaxThreads<T>) k_rows_c2r(RowPassArgs<T> 
         const int c = idx / a.B1, e = idx - c * a.B1;
         const int r0 = r0base + 2 * c, r1 = r0 + 1;
         const cplx<T> z = s[wrap(e - a.c1, n) * P + c];
-        if (r0 < a.nrows) x[(long long)r0 * a.B1 + e] = z.x * a.scale;
-        if (r1 < a.nrows) x[(long long)r1 * a.B1 + e] = z.y * a.scale;
+        if (r0 < a.nrows) x[(long long)r0 * a.B1 + e] = scaled(z.x, a);
+        if (r1 < a.nrows) x[(long long)r1 * a.B1 + e] = scaled(z.y, a);
     }
 }
 

@@ -141,24 +141,46 @@ __device__ __forceinline__ void r32_fft(cplx<T> (&x)[32], cplx<T> *S, int c, int
 {
     using G = R32<N>;
     dft32_regs<T, INV, ZIN>(x);
-    // WN^(t k1) and the exchange: S[k1][t].  The twiddles come from four
-    // loads, WN^(t b) for b = 1..3 and WN^(4t): k1 = 4a + b runs along the chain
-    // of b, one product by WN^(4t) per step (at most 7 products, a few units
-    // in the last place; 31 loads measured 3 % slower over the iteration)
+    // WN^(t k1) and the exchange: S[k1][t].  At 512 and 1024 points the twiddles
+    // come from four loads, WN^(t b) for b = 1..3 and WN^(4t): k1 = 4a + b runs
+    // along the chain of b, one product by WN^(4t) per step (at most 7 products, a
+    // few units in the last place; 31 loads measured 3 % slower over the
+    // iteration).  The shorter lengths take WN^(8t) and WN^(16t) as well and at
+    // most three products: the chains' error, the same in every transform, adds
+    // up over an iteration (50 of a 128^3 object: 2.9e-6 with the chains, 1.3e-6;
+    // F3 at 256 points 31.1 us either way, 33.1 with every twiddle loaded).
     if (sync_in) __syncthreads();  // the buffer may still be read by the previous step
     cplx<T> *Sc = S + c * G::CS;
     const cplx<T> *tt = tw + G::TWT + t;  // tt[k1 P] = WN^(t k1)
-    cplx<T> cur[4] = {__ldg(tt + 4 * G::P), __ldg(tt + G::P), __ldg(tt + 2 * G::P), __ldg(tt + 3 * G::P)};
-    const cplx<T> w4 = cur[0];
+    if constexpr (N >= 512) {
+        cplx<T> cur[4] = {__ldg(tt + 4 * G::P), __ldg(tt + G::P), __ldg(tt + 2 * G::P), __ldg(tt + 3 * G::P)};
+        const cplx<T> w4 = cur[0];
 #pragma unroll
-    for (int k1 = 0; k1 < 32; ++k1) {
-        const int slot = 8 * (k1 & 3) + (k1 >> 2), b = k1 & 3;
-        cplx<T> y = x[slot];
-        if (k1) {
-            y = ctw(y, cur[b], INV);
-            if (k1 + 4 < 32) cur[b] = cmul(cur[b], w4);
+        for (int k1 = 0; k1 < 32; ++k1) {
+            const int slot = 8 * (k1 & 3) + (k1 >> 2), b = k1 & 3;
+            cplx<T> y = x[slot];
+            if (k1) {
+                y = ctw(y, cur[b], INV);
+                if (k1 + 4 < 32) cur[b] = cmul(cur[b], w4);
+            }
+            Sc[k1 * G::ROW + t] = y;
         }
-        Sc[k1 * G::ROW + t] = y;
+    } else {
+        const cplx<T> w4 = __ldg(tt + 4 * G::P), w8 = __ldg(tt + 8 * G::P), w16 = __ldg(tt + 16 * G::P);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            cplx<T> w[8];  // WN^(t (4a + b))
+            w[0] = b ? __ldg(tt + b * G::P) : mk((T)1, (T)0);
+            w[1] = b ? cmul(w[0], w4) : w4;
+            w[2] = b ? cmul(w[0], w8) : w8;
+            w[3] = cmul(w[1], w8);
+            w[4] = b ? cmul(w[0], w16) : w16;
+#pragma unroll
+            for (int a = 5; a < 8; ++a) w[a] = cmul(w[a - 4], w16);
+#pragma unroll
+            for (int a = 0; a < 8; ++a)
+                Sc[(4 * a + b) * G::ROW + t] = a + b ? ctw(x[8 * b + a], w[a], INV) : x[8 * b + a];
+        }
     }
     __syncthreads();
     if constexpr (N <= 256) {
@@ -574,16 +596,16 @@ __global__ void __launch_bounds__(R32<N>::THREADS) k_row_c2r_r32(RowPassArgs<T> 
         if constexpr (ZOUT) {
             if (G::keep(sl)) {
                 const int e = t + G::half_off(G::out_m(sl));
-                if (ok0) xs[(long long)r0 * a.B1 + e] = x[sl].x * a.scale;
-                if (ok1) xs[(long long)r1 * a.B1 + e] = x[sl].y * a.scale;
+                if (ok0) xs[(long long)r0 * a.B1 + e] = scaled(x[sl].x, a);
+                if (ok1) xs[(long long)r1 * a.B1 + e] = scaled(x[sl].y, a);
             }
             continue;
         }
         int e = t + P * G::out_m(sl) + a.c1;
         if (e >= N) e -= N;
         if (e < a.B1) {
-            if (ok0) xs[(long long)r0 * a.B1 + e] = x[sl].x * a.scale;
-            if (ok1) xs[(long long)r1 * a.B1 + e] = x[sl].y * a.scale;
+            if (ok0) xs[(long long)r0 * a.B1 + e] = scaled(x[sl].x, a);
+            if (ok1) xs[(long long)r1 * a.B1 + e] = scaled(x[sl].y, a);
         }
     }
 }

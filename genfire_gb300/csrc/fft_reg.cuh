@@ -504,8 +504,8 @@ __global__ void __launch_bounds__(N / 8 * reg_width<T>(N), kRegMinBlocks<T>) k_r
         int e = reg_final_index<N>(j, k) + a.c1;
         if (e >= N) e -= N;
         if (e < a.B1) {
-            if (r0 < a.nrows) x[(long long)r0 * a.B1 + e] = v[0][k].x * a.scale;
-            if (r1 < a.nrows) x[(long long)r1 * a.B1 + e] = v[0][k].y * a.scale;
+            if (r0 < a.nrows) x[(long long)r0 * a.B1 + e] = scaled(v[0][k].x, a);
+            if (r1 < a.nrows) x[(long long)r1 * a.B1 + e] = scaled(v[0][k].y, a);
         }
     }
 }

@@ -19,14 +19,14 @@ const TwoFixed *two_fixed(int n)
 }
 
 // squared length of the rounded root WR^j, less 1
-static double root_gain(int j, int R)
+double root_gain(int j, int R)
 {
     const double c = (float)root_cos(j, R), s = (float)root_sin(j, R);
     return c * c + s * s - 1.0;
 }
 // an R-point butterfly's: its factors' and the twiddles' between them; of a
 // base radix the mean over its matrix
-static double radix_gain(int R)
+double radix_gain(int R)
 {
     const int A = rdft_split(R), B = R / A;
     double g = 0;

@@ -499,8 +499,8 @@ __device__ __forceinline__ void row_c2r_two(const RowPassArgs<T> &a, const Plan 
 #pragma unroll
         for (int m = 0; m < R; ++m) {
             if (e < cnt) {
-                if (ok0) xs[(long long)r0 * a.B1 + e] = fma(x[m].x, a.scale, x[m].x * a.scale_lo);
-                if (ok1) xs[(long long)(r0 + 1) * a.B1 + e] = fma(x[m].y, a.scale, x[m].y * a.scale_lo);
+                if (ok0) xs[(long long)r0 * a.B1 + e] = scaled(x[m].x, a);
+                if (ok1) xs[(long long)(r0 + 1) * a.B1 + e] = scaled(x[m].y, a);
             }
             e -= tp.R1;
             if (e < 0) e += N;
@@ -556,13 +556,11 @@ template <typename T> bool two_capable(int n)
     return n <= 1024 && make_two_plan(n, p) && (sizeof(T) == 8 || p.R2 <= 16 || two_fixed(n));
 }
 
-// Mean gain (squared length, less 1) of a complex64 transform of n points on
-// this engine, from the rounding of its constants: the rounded root has length
-// 1 + a few 1e-8, and a handful of constants per radix do not average out, so
-// a forward and inverse pair scales the object by 1 + two_gain (300 points:
-// 5e-8).  An iteration leaves the unmeasured frequencies as they are, so over
-// many of them this bias adds up while the roundings' noise does not; the last
-// pass of an inverse transform takes it back (RowPassArgs::scale_lo).
+// Mean gains (squared length, less 1) of complex64 arithmetic, from the rounding
+// of its constants: of the root WR^j, of an R-point butterfly of this engine, of a
+// whole transform of n points on it.
+double root_gain(int j, int R);
+double radix_gain(int R);
 double two_gain(int n);
 
 inline size_t two_row_smem(int nt, int R2, int cp, size_t es) { return (size_t)cp * ((nt + R2 - 1) / R2) * es; }
