@@ -140,8 +140,9 @@ genfire_status genfire_destroy(genfire_ctx *ctx)
     // destructor runs: a delete here, of an incomplete type, would free the
     // object without releasing its device buffers and graph)
     while (!ctx->recons.empty()) gf::recon_destroy(*ctx->recons.begin());
+    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    gf::proj_texture_destroy(ctx->proj_texture);
     if (ctx->stream) {
-        cudaStreamSynchronize(ctx->stream);
         cudaStreamDestroy(ctx->stream);
     }
     delete ctx;

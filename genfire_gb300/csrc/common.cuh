@@ -128,10 +128,14 @@ inline double mround(double x) { return x < 0 ? -std::floor(-x + 0.5) : std::flo
 // The context behind genfire_ctx.  It tracks the reconstructions and batches
 // created on it: genfire_destroy frees whatever is still alive before it
 // destroys the stream they use.
+namespace gf {
+struct ProjTexture;
+}
 struct genfire_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     int sm_count = 0;
+    gf::ProjTexture *proj_texture = nullptr;  // the projector's volume as a texture (project.cu), kept between calls
     int interp = GENFIRE_INTERP_TRILINEAR;  // projector interpolation (genfire_set_projector_interpolation)
     std::string last_error;
     std::set<genfire_recon *> recons;

@@ -143,6 +143,9 @@ void project_batch(genfire_ctx *ctx, int precision, const void *d_vol, int n1, i
                    long long vs1, long long vs2, int P, const double *d_R, void *d_proj,
                    const double *d_measured, double *d_sums, cudaStream_t stream);
 
+// frees a context's projector texture (nullptr: none)
+void proj_texture_destroy(ProjTexture *t);
+
 // Tian_calc_Rfactor_realspace on device buffers: d_model (m1 x m2 x m3),
 // d_projs (p1 x p2 x P double), host angles; Rarr (P) and Rtotal on the host,
 // d_simu (p1 x p2 x P float, optional) on the device.
