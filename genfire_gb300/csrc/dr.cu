@@ -32,6 +32,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <set>
 #include <tuple>
@@ -155,19 +156,19 @@ template <typename T, int N> static void col_reg(const ColPassArgs<T> &a, int ot
     dim3 grid(cdiv(a.ncols, W), other);
     if constexpr (sizeof(T) == 4) {
         if (nc == 2) {
-            k_col_reg<T, N, 2><<<grid, col_threads<T, N, 2>(), reg_smem<T, N>(), st>>>(a);
+            launch_pass(k_col_reg<T, N, 2>, grid, col_threads<T, N, 2>(), reg_smem<T, N>(), st, a);
             return;
         }
     }
-    k_col_reg<T, N, 1><<<grid, col_threads<T, N, 1>(), reg_smem<T, N>(), st>>>(a);
+    launch_pass(k_col_reg<T, N, 1>, grid, col_threads<T, N, 1>(), reg_smem<T, N>(), st, a);
 }
 template <typename T, int N> static void rows_reg(const RowPassArgs<T> &a, bool forward, cudaStream_t st)
 {
     constexpr int W = reg_width<T>(N);
     if (a.W != W) fail(GENFIRE_ERR_STATE, "internal: row tile width mismatch.");
     dim3 grid(cdiv((a.nrows + 1) / 2, W));
-    if (forward) k_row_r2c_reg<T, N><<<grid, N / 8 * W, reg_smem<T, N>(), st>>>(a);
-    else k_row_c2r_reg<T, N><<<grid, N / 8 * W, reg_smem<T, N>(), st>>>(a);
+    if (forward) launch_pass(k_row_r2c_reg<T, N>, grid, N / 8 * W, reg_smem<T, N>(), st, a);
+    else launch_pass(k_row_c2r_reg<T, N>, grid, N / 8 * W, reg_smem<T, N>(), st, a);
 }
 // element offsets along the transform are 32-bit in the register passes
 template <typename T> static bool span_ok(const ColPassArgs<T> &a)
@@ -336,9 +337,9 @@ template <typename T, int N> static void col_r32(const ColPassArgs<T> &a, int ot
     const bool zout = a.out_cnt == N / 2 && a.out_c == N / 4;
     const dim3 grid(cdiv(a.ncols, G::W), other);
     const size_t sm = G::template smem<T>();
-    if (zin && zout) k_col_r32<T, N, true, true><<<grid, G::THREADS, sm, st>>>(a);
-    else if (zout) k_col_r32<T, N, false, true><<<grid, G::THREADS, sm, st>>>(a);
-    else k_col_r32<T, N, false, false><<<grid, G::THREADS, sm, st>>>(a);
+    if (zin && zout) launch_pass(k_col_r32<T, N, true, true>, grid, G::THREADS, sm, st, a);
+    else if (zout) launch_pass(k_col_r32<T, N, false, true>, grid, G::THREADS, sm, st, a);
+    else launch_pass(k_col_r32<T, N, false, false>, grid, G::THREADS, sm, st, a);
 }
 // Launch of k_col_r32_tma: the input as a float tensor {2 in_other, in_dim /
 // in_other, in_cnt} (strides in_other and in_dim complex values), boxes of
@@ -358,7 +359,7 @@ static void col_r32_tma(const ColPassArgs<float> &a, int other, cudaStream_t st)
     if (r != CUDA_SUCCESS) fail(GENFIRE_ERR_CUDA, "tensor map of the fused column pass could not be encoded.");
     const int tiles_x = (int)cdiv(a.ncols, G::W), ntiles = tiles_x * other;
     const int grid = std::min(ntiles, 4 * device_sm_count());
-    k_col_r32_tma<N><<<grid, G::THREADS, r32_tma_smem<N>(), st>>>(a, map, tiles_x, ntiles);
+    launch_pass(k_col_r32_tma<N>, grid, G::THREADS, r32_tma_smem<N>(), st, a, map, tiles_x, ntiles);
 }
 
 template <typename T, int N> static void rows_r32(const RowPassArgs<T> &a, bool forward, cudaStream_t st)
@@ -368,11 +369,11 @@ template <typename T, int N> static void rows_r32(const RowPassArgs<T> &a, bool 
     const size_t sm = G::template smem<T>();
     const bool half = a.B1 == N / 2 && a.c1 == N / 4;  // the centred half of the row
     if (forward) {
-        if (half) k_row_r2c_r32<T, N, true><<<grid, G::THREADS, sm, st>>>(a);
-        else k_row_r2c_r32<T, N, false><<<grid, G::THREADS, sm, st>>>(a);
+        if (half) launch_pass(k_row_r2c_r32<T, N, true>, grid, G::THREADS, sm, st, a);
+        else launch_pass(k_row_r2c_r32<T, N, false>, grid, G::THREADS, sm, st, a);
     } else {
-        if (half) k_row_c2r_r32<T, N, true><<<grid, G::THREADS, sm, st>>>(a);
-        else k_row_c2r_r32<T, N, false><<<grid, G::THREADS, sm, st>>>(a);
+        if (half) launch_pass(k_row_c2r_r32<T, N, true>, grid, G::THREADS, sm, st, a);
+        else launch_pass(k_row_c2r_r32<T, N, false>, grid, G::THREADS, sm, st, a);
     }
 }
 
@@ -400,7 +401,7 @@ template <typename T> static void launch_colpass(ColPassArgs<T> a, int other, cu
     } else if (variant == kColGeneric) {
         const size_t sm = tile_smem<T>(a.pl.n, a.W);
         dim3 grid(cdiv(a.ncols, a.W), other);
-        k_colpass<T><<<grid, tile_threads(a.pl.n, a.W), sm, st>>>(a);
+        launch_pass(k_colpass<T>, grid, tile_threads(a.pl.n, a.W), sm, st, a);
     } else {
         col_reg_any<T>(a, other, st, variant == kColReg2 ? 2 : 1);
     }
@@ -500,8 +501,8 @@ template <typename T> static void launch_rows(RowPassArgs<T> a, bool forward, cu
         const size_t sm = tile_smem<T>(a.pl.n, a.W);
         const int pairs = (a.nrows + 1) / 2;
         dim3 grid(cdiv(pairs, a.W));
-        if (forward) k_rows_r2c<T><<<grid, tile_threads(a.pl.n, a.W), sm, st>>>(a);
-        else k_rows_c2r<T><<<grid, tile_threads(a.pl.n, a.W), sm, st>>>(a);
+        if (forward) launch_pass(k_rows_r2c<T>, grid, tile_threads(a.pl.n, a.W), sm, st, a);
+        else launch_pass(k_rows_c2r<T>, grid, tile_threads(a.pl.n, a.W), sm, st, a);
     }
     GF_CHECK_LAUNCH();
 }
@@ -1069,8 +1070,6 @@ __global__ void k_extract(const T *const *__restrict__ xs, const Ctl *__restrict
 struct ReconBase {
     virtual ~ReconBase() {}
     virtual void iterate(int count) = 0;
-    // one iteration as a (not instantiated) graph, for batches
-    virtual cudaGraph_t capture_iteration() = 0;
     // one iteration's launches on st (for a caller's own capture), the kernel
     // attributes that must be set before a capture, and the grid size (the
     // batch orders members by it)
@@ -1087,6 +1086,10 @@ struct ReconBase {
     virtual void set_rfree(int nshells, const int64_t *counts, const int64_t *indices) = 0;
     virtual int rfree(double *out) const = 0;
 };
+
+// iterations of the long graph, and the count of a call from which it is made
+// (making it costs 0.2 ms, a launch of its own per iteration 3 us)
+constexpr int kLongGraph = 4, kLongGraphFrom = 96;
 
 template <typename T> struct ReconT : ReconBase {
     genfire_ctx *ctx;
@@ -1105,13 +1108,20 @@ template <typename T> struct ReconT : ReconBase {
     double denom = 0;
     int it_done = 0;
     int vF2 = kColAuto, vF3 = kColAuto, vI2 = kColAuto;  // column-pass variants (autotuned)
-    cudaGraphExec_t exec = nullptr;
+    cudaGraphExec_t exec = nullptr;       // one iteration
+    cudaGraphExec_t exec_long = nullptr;  // kLongGraph iterations, made by the first call that runs several of them
     std::vector<double> errR, Rarr, Rarr2;
 
     ~ReconT() override
     {
-        if (exec) cudaGraphExecDestroy(exec);
+        drop_graphs();
         cudaStreamSynchronize(ctx->stream);
+    }
+    void drop_graphs()
+    {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (exec_long) cudaGraphExecDestroy(exec_long);
+        exec = exec_long = nullptr;
     }
 
     void setup(const void *Min, const uint8_t *maskin, const uint8_t *support, const void *initial,
@@ -1479,30 +1489,30 @@ template <typename T> struct ReconT : ReconBase {
     void prepare_capture() override { ensure_smem_attrs<T>(); }
     long long grid_points() const override { return (long long)n1 * n2 * n1; }
 
-    cudaGraph_t capture_iteration() override
+    // count iterations as one graph
+    cudaGraphExec_t make_graph(int count)
     {
         cudaStream_t st = ctx->stream;
         ensure_smem_attrs<T>();  // kernel attributes are set outside the capture
         cudaGraph_t graph = nullptr;
         GF_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         try {
-            enqueue_iteration(st);
+            std::unique_ptr<PassOverlap> overlap(count > 1 ? new PassOverlap : nullptr);
+            for (int i = 0; i < count; ++i) enqueue_iteration(st);
         } catch (...) {
             cudaStreamEndCapture(st, &graph);
             if (graph) cudaGraphDestroy(graph);
             throw;
         }
         GF_CUDA(cudaStreamEndCapture(st, &graph));
-        return graph;
+        cudaGraphExec_t e = nullptr;
+        const cudaError_t err = cudaGraphInstantiate(&e, graph, 0);
+        cudaGraphDestroy(graph);
+        GF_CUDA(err);
+        return e;
     }
 
-    void build_graph()
-    {
-        cudaGraph_t graph = capture_iteration();
-        cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
-        cudaGraphDestroy(graph);
-        GF_CUDA(e);
-    }
+    void build_graph() { exec = make_graph(1); }
 
     // Rfree monitor (reconstruct.m:46-69, :137-146): withheld points of each
     // shell as 0-based linear indices into the centred grid; the caller has
@@ -1567,10 +1577,7 @@ template <typename T> struct ReconT : ReconBase {
         GF_CUDA(cudaStreamSynchronize(st));
         nshells = nsh;
         nrfree = tot;
-        if (exec) {
-            cudaGraphExecDestroy(exec);
-            exec = nullptr;
-        }
+        drop_graphs();
         build_graph();
     }
     // Rfree(shell, iteration) for the iterations run so far, column-major
@@ -1627,10 +1634,24 @@ template <typename T> struct ReconT : ReconBase {
         if (count < 0 || it_done + count > p.numIterations)
             fail(GENFIRE_ERR_STATE, "iterate: more iterations requested than numIterations.");
         cudaStream_t st = ctx->stream;
-        for (int i = 0; i < count; ++i) {
-            GF_CUDA(cudaGraphLaunch(exec, st));
-            ++it_done;
-            if (p.monitor_R == 1 && it_done % p.monitorR_loopLength == 0) monitor();
+        // kLongGraph iterations per launch where as many are left before the next
+        // stop (the R-factor monitor's): a launch of its own per iteration leaves a
+        // gap between them (200 iterations of a 64^3 object: 5.29 ms, 4.69 with the
+        // passes overlapped as well; see launch_pass)
+        const int stop = p.monitor_R == 1 ? p.monitorR_loopLength : 0;
+        for (int left = count; left > 0;) {
+            const int run = stop ? std::min(left, stop - it_done % stop) : left;
+            if (run >= kLongGraph && (exec_long || left >= kLongGraphFrom)) {
+                if (!exec_long) exec_long = make_graph(kLongGraph);
+                GF_CUDA(cudaGraphLaunch(exec_long, st));
+                it_done += kLongGraph;
+                left -= kLongGraph;
+            } else {
+                GF_CUDA(cudaGraphLaunch(exec, st));
+                ++it_done;
+                --left;
+            }
+            if (stop && it_done % stop == 0) monitor();
         }
         GF_CUDA(cudaStreamSynchronize(st));
         check_device_error();

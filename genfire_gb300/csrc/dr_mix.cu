@@ -56,6 +56,7 @@ __device__ __forceinline__ void mix_final(cplx<T> (&v)[N1][8], int j, const cplx
 template <typename T, int N2, int N1>
 __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_col_mix(ColPassArgs<T> a)
 {
+    pass_begin();
     constexpr int N = N1 * N2;
     constexpr int W = mix_width<T>(N);
     using Lay = ColLayout<N2, W * N1>;
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_col_mix(ColPassArg
 template <typename T, int N2, int N1>
 __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_row_r2c_mix(RowPassArgs<T> a)
 {
+    pass_begin();
     constexpr int N = N1 * N2;
     constexpr int W = mix_width<T>(N);
     constexpr int TPC = N2 / 8;
@@ -189,6 +191,7 @@ __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_row_r2c_mix(RowPas
 template <typename T, int N2, int N1>
 __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_row_c2r_mix(RowPassArgs<T> a)
 {
+    pass_begin();
     constexpr int N = N1 * N2;
     constexpr int W = mix_width<T>(N);
     constexpr int TPC = N2 / 8;
@@ -311,7 +314,7 @@ template <typename T> bool launch_col_mix(const ColPassArgs<T> &a, int other, cu
     if (a.W != mix_width<T>(a.pl.n)) fail(GENFIRE_ERR_STATE, "internal: mixed-radix tile width mismatch.");
     ensure_mix_attrs<T>();
     const dim3 grid(cdiv(a.ncols, a.W), other);
-#define GF_COL(n2, n1) k_col_mix<T, n2, n1><<<grid, mix_threads<T, n2, n1>(), mix_smem<T, n2, n1>(), st>>>(a)
+#define GF_COL(n2, n1) launch_pass(k_col_mix<T, n2, n1>, grid, mix_threads<T, n2, n1>(), mix_smem<T, n2, n1>(), st, a)
     GF_MIX_CASES(GF_COL)
 #undef GF_COL
     return false;
@@ -327,8 +330,8 @@ template <typename T> bool launch_rows_mix(const RowPassArgs<T> &a, bool forward
     const dim3 grid(cdiv((a.nrows + 1) / 2, a.W));
 #define GF_ROW(n2, n1)                                                                                    \
     do {                                                                                                  \
-        if (forward) k_row_r2c_mix<T, n2, n1><<<grid, mix_threads<T, n2, n1>(), mix_smem<T, n2, n1>(), st>>>(a); \
-        else k_row_c2r_mix<T, n2, n1><<<grid, mix_threads<T, n2, n1>(), mix_smem<T, n2, n1>(), st>>>(a);  \
+        if (forward) launch_pass(k_row_r2c_mix<T, n2, n1>, grid, mix_threads<T, n2, n1>(), mix_smem<T, n2, n1>(), st, a); \
+        else launch_pass(k_row_c2r_mix<T, n2, n1>, grid, mix_threads<T, n2, n1>(), mix_smem<T, n2, n1>(), st, a);  \
     } while (0)
     GF_MIX_CASES(GF_ROW)
 #undef GF_ROW

@@ -306,6 +306,7 @@ __device__ __forceinline__ void col_r32_tile(const ColPassArgs<T> &a, cplx<T> *s
 template <typename T, int N, bool ZIN, bool ZOUT>
 __global__ void __launch_bounds__(R32<N>::THREADS, r32_col_min_blocks(N)) k_col_r32(ColPassArgs<T> a)
 {
+    pass_begin();
     using G = R32<N>;
     constexpr int P = G::P, W = G::W;
     using Lay = typename G::Lay;
@@ -415,6 +416,7 @@ template <int N>
 __global__ void __launch_bounds__(R32<N>::THREADS, 4)
     k_col_r32_tma(ColPassArgs<float> a, const __grid_constant__ CUtensorMap tmap, int tiles_x, int ntiles)
 {
+    pass_begin();
     using G = R32<N>;
     constexpr int W = G::W;
     constexpr uint32_t kBytes = r32_tma_stage_bytes<N>();
@@ -476,6 +478,7 @@ constexpr int kRowLoadGroup = 8;
 template <typename T, int N, bool ZIN>
 __global__ void __launch_bounds__(R32<N>::THREADS) k_row_r2c_r32(RowPassArgs<T> a)
 {
+    pass_begin();
     using G = R32<N>;
     constexpr int P = G::P, W = G::W;
     using RowLay = typename G::RowLay;
@@ -551,6 +554,7 @@ __global__ void __launch_bounds__(R32<N>::THREADS) k_row_r2c_r32(RowPassArgs<T> 
 template <typename T, int N, bool ZOUT>
 __global__ void __launch_bounds__(R32<N>::THREADS) k_row_c2r_r32(RowPassArgs<T> a)
 {
+    pass_begin();
     using G = R32<N>;
     constexpr int P = G::P, W = G::W;
     // the CTA's rows hold no support voxel: the next forward pass treats them

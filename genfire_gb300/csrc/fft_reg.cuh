@@ -309,6 +309,7 @@ __device__ __forceinline__ void st_global(cplx<T> *p, const cplx<T> (&v)[NC][8],
 template <typename T, int N, int NC>
 __global__ void __launch_bounds__(col_threads<T, N, NC>(), kRegMinBlocks<T>) k_col_reg(ColPassArgs<T> a)
 {
+    pass_begin();
     constexpr int W = reg_width<T>(N);
     constexpr int WT = W / NC;  // threads across the tile's columns
     using Lay = ColLayout<N, W>;
@@ -422,6 +423,7 @@ __device__ __forceinline__ void load_row_pair(const RowPassArgs<T> &a, const T *
 template <typename T, int N>
 __global__ void __launch_bounds__(N / 8 * reg_width<T>(N), kRegMinBlocks<T>) k_row_r2c_reg(RowPassArgs<T> a)
 {
+    pass_begin();
     constexpr int W = reg_width<T>(N);
     constexpr int TPC = N / 8;
     using Lay = RowLayout<N, W>;
@@ -461,6 +463,7 @@ __global__ void __launch_bounds__(N / 8 * reg_width<T>(N), kRegMinBlocks<T>) k_r
 template <typename T, int N>
 __global__ void __launch_bounds__(N / 8 * reg_width<T>(N), kRegMinBlocks<T>) k_row_c2r_reg(RowPassArgs<T> a)
 {
+    pass_begin();
     constexpr int W = reg_width<T>(N);
     constexpr int TPC = N / 8;
     using Lay = RowLayout<N, W>;

@@ -345,6 +345,7 @@ __device__ __noinline__ void two_transform(const ColPassArgs<T> &a, const Plan &
 template <typename T, int RMAX, class Plan>
 __device__ __forceinline__ void col_two(const ColPassArgs<T> &a, const Plan &tp, int lw)
 {
+    pass_begin();
     if (a.ctl && blockIdx.x == 0 && blockIdx.y == 0) ctl_mid_update(a.ctl, a.partial, a.nparts, a.denom, a.hist);
     const bool both = (a.mode & 3) == 3;
     if (a.mode & 1) two_transform<T, RMAX>(a, tp, lw, 0, false, !both);
@@ -382,6 +383,7 @@ __global__ void __launch_bounds__(two_fixed_threads(R2, two_width<T>(R1 * R2)), 
 template <typename T, int RMAX, class Plan>
 __device__ __forceinline__ void row_r2c_two(const RowPassArgs<T> &a, const Plan &tp, int cp)
 {
+    pass_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (a.ctl && blockIdx.x == 0 && threadIdx.x == 0) ctl_begin_update(a.ctl, a.changes);
     if (row_pairs_empty(a, a.W)) {
@@ -453,6 +455,7 @@ __device__ __forceinline__ void row_r2c_two(const RowPassArgs<T> &a, const Plan 
 template <typename T, int RMAX, class Plan>
 __device__ __forceinline__ void row_c2r_two(const RowPassArgs<T> &a, const Plan &tp, int cp)
 {
+    pass_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (row_pairs_empty(a, a.W)) return;
     const int N = tp.N;
@@ -572,13 +575,13 @@ template <int R1, int R2> TwoFixed make_two_fixed()
     TwoFixed f;
     f.n = P::N;
     f.col = [](const ColPassArgs<float> &a, int other, cudaStream_t st) {
-        k_col_fixed<float, R1, R2><<<dim3(cdiv(a.ncols, W), other), NT, (size_t)two_tile(P{}) * W * sizeof(float2), st>>>(a);
+        launch_pass(k_col_fixed<float, R1, R2>, dim3(cdiv(a.ncols, W), other), NT, (size_t)two_tile(P{}) * W * sizeof(float2), st, a);
     };
     f.rows = [](const RowPassArgs<float> &a, bool forward, cudaStream_t st) {
         const dim3 grid(cdiv((a.nrows + 1) / 2, W));
         const size_t sm = two_row_smem(NT, R2, two_fixed_cp<R1, R2>(), sizeof(float2));
-        if (forward) k_row_r2c_fixed<float, R1, R2><<<grid, NT, sm, st>>>(a);
-        else k_row_c2r_fixed<float, R1, R2><<<grid, NT, sm, st>>>(a);
+        if (forward) launch_pass(k_row_r2c_fixed<float, R1, R2>, grid, NT, sm, st, a);
+        else launch_pass(k_row_c2r_fixed<float, R1, R2>, grid, NT, sm, st, a);
     };
     return f;
 }
@@ -598,8 +601,8 @@ template <typename T> bool launch_col_two_impl(const ColPassArgs<T> &a, int othe
     }
     const dim3 grid(cdiv(a.ncols, a.W), other);
     const size_t sm = (size_t)two_tile(p) * a.W * sizeof(cplx<T>);
-    if (p.R2 <= 16) k_col_two<T, 16><<<grid, two_threads(p, a.W), sm, st>>>(a, p, lw);
-    else if constexpr (sizeof(T) == 8) k_col_two<T, 32><<<grid, two_threads(p, a.W), sm, st>>>(a, p, lw);
+    if (p.R2 <= 16) launch_pass(k_col_two<T, 16>, grid, two_threads(p, a.W), sm, st, a, p, lw);
+    else if constexpr (sizeof(T) == 8) launch_pass(k_col_two<T, 32>, grid, two_threads(p, a.W), sm, st, a, p, lw);
     return true;
 }
 template <typename T> bool launch_rows_two_impl(const RowPassArgs<T> &a, bool forward, cudaStream_t st)
@@ -616,11 +619,11 @@ template <typename T> bool launch_rows_two_impl(const RowPassArgs<T> &a, bool fo
     const int cp = two_tile(p) | 1, nt = two_threads(p, a.W);
     const size_t sm = two_row_smem(nt, p.R2, cp, sizeof(cplx<T>));
     if (p.R2 <= 16) {
-        if (forward) k_row_r2c_two<T, 16><<<grid, nt, sm, st>>>(a, p, cp);
-        else k_row_c2r_two<T, 16><<<grid, nt, sm, st>>>(a, p, cp);
+        if (forward) launch_pass(k_row_r2c_two<T, 16>, grid, nt, sm, st, a, p, cp);
+        else launch_pass(k_row_c2r_two<T, 16>, grid, nt, sm, st, a, p, cp);
     } else if constexpr (sizeof(T) == 8) {
-        if (forward) k_row_r2c_two<T, 32><<<grid, nt, sm, st>>>(a, p, cp);
-        else k_row_c2r_two<T, 32><<<grid, nt, sm, st>>>(a, p, cp);
+        if (forward) launch_pass(k_row_r2c_two<T, 32>, grid, nt, sm, st, a, p, cp);
+        else launch_pass(k_row_c2r_two<T, 32>, grid, nt, sm, st, a, p, cp);
     }
     return true;
 }
