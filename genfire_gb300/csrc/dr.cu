@@ -841,7 +841,10 @@ __global__ void k_tab_write(const cplx<T> *__restrict__ M, const uint8_t *__rest
     for (int q3 = seg * kTabSeg; q3 < e3; ++q3) {
         TabEntry<T> e;
         double am;
-        if (tab_point<T, true>(M, mask, g, q1, q2, q3, e, am)) tab[o++] = e;
+        if (tab_point<T, true>(M, mask, g, q1, q2, q3, e, am)) {
+            e.set_abs();
+            tab[o++] = e;
+        }
     }
 }
 

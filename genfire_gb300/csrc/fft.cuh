@@ -213,6 +213,18 @@ template <typename T> struct Dft<3, T> {
     }
 };
 
+template <> struct Dft<3, double> {
+    static __device__ __forceinline__ void run(double2 *v, bool inv, const double2 *, int)
+    {
+        const double s3 = inv ? -0.86602540378443864676 : 0.86602540378443864676;
+        const double2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+        const double2 a = mk(fma(-0.5, t.x, v[0].x), fma(-0.5, t.y, v[0].y));
+        v[0] = cadd(v[0], t);
+        v[1] = mk(fma(s3, d.y, a.x), fma(-s3, d.x, a.y));
+        v[2] = mk(fma(-s3, d.y, a.x), fma(s3, d.x, a.y));
+    }
+};
+
 template <typename T> struct Dft<5, T> {
     static __device__ __forceinline__ void run(cplx<T> *v, bool inv, const cplx<T> *, int)
     {
@@ -333,6 +345,23 @@ template <typename T> struct TabEntry {
     uint32_t cmq;     // bit c: -q in C while delay index c is in force
     cplx<T> Mq;       // measuredK(q)
     cplx<T> Mmq;      // measuredK(-q)
+    __device__ __forceinline__ T abs_q() const { return sqrt(Mq.x * Mq.x + Mq.y * Mq.y); }
+    __device__ __forceinline__ T abs_mq() const { return sqrt(Mmq.x * Mmq.x + Mmq.y * Mmq.y); }
+    __device__ __forceinline__ void set_abs() {}
+};
+// complex128: the magnitudes are stored, since a square root takes as many FP64
+// instructions as half a radix-4 butterfly and every iteration needs them again
+template <> struct TabEntry<double> {
+    uint32_t pos, eflags, cq, cmq;
+    double2 Mq, Mmq;
+    double aq, amq;
+    __device__ __forceinline__ double abs_q() const { return aq; }
+    __device__ __forceinline__ double abs_mq() const { return amq; }
+    __device__ __forceinline__ void set_abs()
+    {
+        aq = sqrt(Mq.x * Mq.x + Mq.y * Mq.y);
+        amq = sqrt(Mmq.x * Mmq.x + Mmq.y * Mmq.y);
+    }
 };
 
 // ---------------------------------------------------------------------------
@@ -567,12 +596,10 @@ __global__ void __launch_bounds__(kTileMaxThreads<T>) k_colpass(ColPassArgs<T> a
             cplx<T> k = s[q3 * P + cl];
             const T mk_ = sqrt(k.x * k.x + k.y * k.y);
             if (t.eflags & 1u) {
-                const T mq = sqrt(t.Mq.x * t.Mq.x + t.Mq.y * t.Mq.y);
-                acc += fabs((double)mk_ - (double)mq);
+                acc += fabs((double)mk_ - (double)t.abs_q());
             }
             if (t.eflags & 2u) {
-                const T mm = sqrt(t.Mmq.x * t.Mmq.x + t.Mmq.y * t.Mmq.y);
-                acc += fabs((double)mk_ - (double)mm);
+                acc += fabs((double)mk_ - (double)t.abs_mq());
             }
             const bool eq = (t.cq >> ci) & 1u, emq = (t.cmq >> ci) & 1u;
             if (eq || emq) {
