@@ -20,7 +20,6 @@
 // the same centred box), so the forward passes skip the zero rows and the
 // inverse passes only produce the box.
 #include <cub/cub.cuh>
-#include <cudaTypedefs.h>  // PFN_cuTensorMapEncodeTiled_v12000
 
 #include "fft.cuh"
 #include "fft_reg.cuh"
@@ -128,8 +127,8 @@ template <typename T, int N> static void set_reg_attrs()
 // mixed-radix engine, the radix-32 engines for 512 and 1024 complex64 points
 // (fft_r32.cuh: 32 x 16 and 32 x 32, one exchange per transform), the two-stage
 // engine for lengths that split into two factors up to 32, and for the
-// fused 512-point pass the persistent radix-32 pass fed by TMA tensor copies
-// (measured 6 % slower than variant 4 on the 512^3 iteration; an autotuner
+// fused 512-point pass the persistent radix-32 pass fed by bulk copies
+// (0.206 ms against variant 4's 0.186 in the 512^3 iteration; an autotuner
 // candidate).
 enum ColVariant { kColAuto = -1, kColGeneric = 0, kColReg1 = 1, kColReg2 = 2, kColMix = 3, kColR32 = 4, kColR32Tma = 5, kColTwo = 6 };
 
@@ -145,7 +144,7 @@ template <typename T> static bool pair_capable(const ColPassArgs<T> &a)
 {
     auto al = [](const void *p) { return ((uintptr_t)p & 15u) == 0; };
     return sizeof(T) == 4 && a.col_stride == 1 && al(a.in) && al(a.out) && a.in_dim % 2 == 0 &&
-           a.in_other % 2 == 0 && a.out_dim % 2 == 0 && a.out_other % 2 == 0;
+           a.in_other % 2 == 0 && a.out_dim % 2 == 0 && a.out_other % 2 == 0 && a.in_blk % 2 == 0 && a.out_blk % 2 == 0;
 }
 
 // Register-resident passes for power-of-two lengths 64..1024.
@@ -243,22 +242,6 @@ static int r32_width(int n)
     }
 }
 
-// The driver's tensor-map encoder (cuTensorMapEncodeTiled), through the
-// runtime's entry-point query so the library needs no link to libcuda.
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
-{
-    static std::once_flag once;
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    std::call_once(once, [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    });
-    return fn;
-}
-
 static int device_sm_count()
 {
     static std::mutex mu;
@@ -274,10 +257,9 @@ static int device_sm_count()
     return n;
 }
 
-// The persistent, TMA-fed fused 512-point pass (k_col_r32_tma): complex64, the
-// centred half of a box in and out, unit column stride, tiles inside the rows
-// of the input, strides that a tensor map can describe.
-template <typename T> static bool tma_capable(const ColPassArgs<T> &a, int other)
+// The persistent fused 512-point pass fed by bulk copies (k_col_r32_tma):
+// complex64, the centred half of a box in and out, the rows of a tile in one piece.
+template <typename T> static bool tma_capable(const ColPassArgs<T> &a)
 {
     if constexpr (sizeof(T) != 4) {
         return false;
@@ -285,17 +267,15 @@ template <typename T> static bool tma_capable(const ColPassArgs<T> &a, int other
         constexpr int N = 512, W = R32<N>::W;
         if (a.pl.n != N || !(a.mode & 1) || !(a.mode & 2) || a.col_stride != 1 || a.W != W) return false;
         if (!(a.in_cnt == N / 2 && a.in_c == N / 4 && a.out_cnt == N / 2 && a.out_c == N / 4)) return false;
-        if (((uintptr_t)a.in & 15u) != 0 || a.in_other <= 0 || a.in_dim % a.in_other != 0) return false;
-        if ((a.in_other * 8) % 16 != 0 || (a.in_dim * 8) % 16 != 0) return false;
-        if ((long long)cdiv(a.ncols, W) * W > a.in_other || other > a.in_dim / a.in_other) return false;
-        return span_ok(a) && tensor_map_encoder() != nullptr;
+        if (a.in_dim != W || a.blk != 0 || a.in_blk < N / 2 * W || a.in_other < N / 2 * W) return false;
+        return ((uintptr_t)a.in & 15u) == 0 && a.in_blk % 2 == 0 && a.in_other % 2 == 0;
     }
 }
 
-template <typename T> static bool col_variant_ok(const ColPassArgs<T> &a, int v, int other = 1)
+template <typename T> static bool col_variant_ok(const ColPassArgs<T> &a, int v)
 {
     if (v == kColGeneric) return true;
-    if (v == kColR32Tma) return tma_capable(a, other);
+    if (v == kColR32Tma) return tma_capable(a);
     if (v == kColR32)
         return sizeof(T) == 4 && r32_width(a.pl.n) > 0 && span_ok(a) && (!(a.mode & 4) || a.W == r32_width(a.pl.n));
     if (v == kColMix) return span_ok(a) && mix_capable<T>(a.pl.n);
@@ -341,25 +321,14 @@ template <typename T, int N> static void col_r32(const ColPassArgs<T> &a, int ot
     else if (zout) launch_pass(k_col_r32<T, N, false, true>, grid, G::THREADS, sm, st, a);
     else launch_pass(k_col_r32<T, N, false, false>, grid, G::THREADS, sm, st, a);
 }
-// Launch of k_col_r32_tma: the input as a float tensor {2 in_other, in_dim /
-// in_other, in_cnt} (strides in_other and in_dim complex values), boxes of
-// {2 W, 1, N/2}; a persistent grid of 4 CTAs per SM.
+// Launch of k_col_r32_tma: a persistent grid of 4 CTAs per SM.
 static void col_r32_tma(const ColPassArgs<float> &a, int other, cudaStream_t st)
 {
     constexpr int N = 512;
     using G = R32<N>;
-    CUtensorMap map;
-    const cuuint64_t dims[3] = {(cuuint64_t)(2 * a.in_other), (cuuint64_t)(a.in_dim / a.in_other), (cuuint64_t)a.in_cnt};
-    const cuuint64_t strides[2] = {(cuuint64_t)(a.in_other * 8), (cuuint64_t)(a.in_dim * 8)};
-    const cuuint32_t box[3] = {2 * G::W, 1, N / 2};
-    const cuuint32_t es[3] = {1, 1, 1};
-    const CUresult r = tensor_map_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<cplx<float> *>(a.in), dims,
-                                            strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) fail(GENFIRE_ERR_CUDA, "tensor map of the fused column pass could not be encoded.");
     const int tiles_x = (int)cdiv(a.ncols, G::W), ntiles = tiles_x * other;
     const int grid = std::min(ntiles, 4 * device_sm_count());
-    launch_pass(k_col_r32_tma<N>, grid, G::THREADS, r32_tma_smem<N>(), st, a, map, tiles_x, ntiles);
+    launch_pass(k_col_r32_tma<N>, grid, G::THREADS, r32_tma_smem<N>(), st, a, tiles_x, ntiles);
 }
 
 template <typename T, int N> static void rows_r32(const RowPassArgs<T> &a, bool forward, cudaStream_t st)
@@ -380,9 +349,11 @@ template <typename T, int N> static void rows_r32(const RowPassArgs<T> &a, bool 
 template <typename T> static void launch_colpass(ColPassArgs<T> a, int other, cudaStream_t st, int variant = kColAuto)
 {
     a.P = a.W + 1;
+    if (!a.in_blk) a.in_blk = (long long)(a.W << a.blk) * a.col_stride;
+    if (!a.out_blk) a.out_blk = (long long)(a.W << a.blk) * a.col_stride;
     const int forced = forced_col_variant();
-    if (forced != kColAuto && col_variant_ok(a, forced, other)) variant = forced;
-    if (variant == kColAuto || !col_variant_ok(a, variant, other)) variant = default_col_variant(a);
+    if (forced != kColAuto && col_variant_ok(a, forced)) variant = forced;
+    if (variant == kColAuto || !col_variant_ok(a, variant)) variant = default_col_variant(a);
     if (variant == kColR32Tma) {
         if constexpr (sizeof(T) == 4) col_r32_tma(a, other, st);
     } else if (variant == kColR32) {
@@ -421,12 +392,12 @@ template <typename T> static int autotune_colpass(ColPassArgs<T> a, int other, c
     ensure_smem_attrs<T>();
     {
         const int f = forced_col_variant();
-        if (f != kColAuto && col_variant_ok(a, f, other)) return f;
+        if (f != kColAuto && col_variant_ok(a, f)) return f;
     }
     int dev = 0;
     GF_CUDA(cudaGetDevice(&dev));
     const std::vector<long long> key = {dev, (long long)sizeof(T), a.pl.n, a.mode, a.ncols, other, a.in_cnt,
-                                        a.in_c, a.out_cnt, a.out_c, a.in_dim, a.in_other, a.out_dim, a.out_other};
+                                        a.in_c, a.out_cnt, a.out_c, a.in_dim, a.in_other, a.out_dim, a.out_other, a.in_blk, a.out_blk, a.blk};
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
@@ -440,7 +411,7 @@ template <typename T> static int autotune_colpass(ColPassArgs<T> a, int other, c
     int best = kColAuto;
     float best_ms = 0, default_ms = -1;
     for (int v : {kColGeneric, kColReg1, kColReg2, kColMix, kColR32, kColR32Tma, kColTwo}) {
-        if (!col_variant_ok(a, v, other)) continue;
+        if (!col_variant_ok(a, v)) continue;
         launch_colpass<T>(a, other, st, v);
         GF_CUDA(cudaEventRecord(e0, st));
         for (int r = 0; r < 3; ++r) launch_colpass<T>(a, other, st, v);
@@ -1310,12 +1281,33 @@ template <typename T> struct ReconT : ReconBase {
         build_graph();
     }
 
+    // Y2 is stored as [q1 block][q2][z][q1 in the block], a block being the
+    // wider of the two passes' tiles: what a CTA of the dim-3 pass reads and
+    // writes is one piece of memory (or a regular part of one) instead of B3
+    // pieces of 32 or 64 bytes, B2 ld1 elements apart.  The dim-2 passes, whose
+    // pieces lay one grid row apart, now take them B3 block rows apart.  Measured,
+    // rows [z][q2][q1] against this, complex64 in ms (F2 F3 I2, iteration):
+    //   1024^3  0.54 2.63 0.42, 3.97     0.64 1.51 0.46, 2.98
+    //    768^3  0.50 1.36 0.58, 2.76     0.53 1.03 0.54, 2.42
+    //    512^3  0.068 0.200 0.052, 0.368  0.071 0.186 0.058, 0.363
+    //    256^3  0.016 0.031 0.015, 0.070  the same; complex128 the same (FP64 pipe)
+    // Blocks of 16 and 32 columns: 1.77 for F3 at 1024^3.
+    void y2_strides(ColPassArgs<T> &a, long long &dim2, long long &dim3, long long &blk) const
+    {
+        const int Q = std::max(W2, W3);
+        dim3 = Q;
+        dim2 = (long long)Q * B3;
+        blk = dim2 * n2;
+        a.blk = 0;
+        while ((a.W << a.blk) < Q) ++a.blk;
+    }
     // F2: dim 2 forward, box rows in, all n2 frequencies out
     ColPassArgs<T> f2_args()
     {
         ColPassArgs<T> a = colargs<T>(pl2, tw2, W2, h1);
         a.in = Y1.as<cplx<T>>(); a.in_dim = ld1; a.in_other = (long long)ld1 * B2; a.in_cnt = B2; a.in_c = B2 / 2;
-        a.out = Y2.as<cplx<T>>(); a.out_dim = ld1; a.out_other = (long long)ld1 * n2; a.out_cnt = n2; a.out_c = 0;
+        a.out = Y2.as<cplx<T>>(); a.out_cnt = n2; a.out_c = 0;
+        y2_strides(a, a.out_dim, a.out_other, a.out_blk);
         a.mode = 1;
         a.zmask = zmask.as<uint8_t>();  // zero slabs stay zero (nullptr when not built)
         a.zmask_zero = 1;
@@ -1326,8 +1318,10 @@ template <typename T> struct ReconT : ReconBase {
     {
         Ctl *c = ctl.as<Ctl>();
         ColPassArgs<T> b = colargs<T>(pl1, tw1, W3, h1);
-        b.in = Y2.as<cplx<T>>(); b.in_dim = (long long)ld1 * n2; b.in_other = ld1; b.in_cnt = B3; b.in_c = B3 / 2;
-        b.out = Y2.as<cplx<T>>(); b.out_dim = (long long)ld1 * n2; b.out_other = ld1; b.out_cnt = B3; b.out_c = B3 / 2;
+        b.in = Y2.as<cplx<T>>(); b.in_cnt = B3; b.in_c = B3 / 2;
+        b.out = Y2.as<cplx<T>>(); b.out_cnt = B3; b.out_c = B3 / 2;
+        y2_strides(b, b.in_other, b.in_dim, b.in_blk);
+        y2_strides(b, b.out_other, b.out_dim, b.out_blk);
         b.mode = 1 | 2 | 4;
         b.tab_off = taboff.as<int>(); b.tab = tab.as<TabEntry<T>>(); b.h1 = h1; b.partial = partial.as<double>();
         b.err = errf.as<int>();
@@ -1344,7 +1338,8 @@ template <typename T> struct ReconT : ReconBase {
     ColPassArgs<T> i2_args(bool with_ctl = true)
     {
         ColPassArgs<T> d = colargs<T>(pl2, tw2, W2, h1);
-        d.in = Y2.as<cplx<T>>(); d.in_dim = ld1; d.in_other = (long long)ld1 * n2; d.in_cnt = n2; d.in_c = 0;
+        d.in = Y2.as<cplx<T>>(); d.in_cnt = n2; d.in_c = 0;
+        y2_strides(d, d.in_dim, d.in_other, d.in_blk);
         d.out = Y1.as<cplx<T>>(); d.out_dim = ld1; d.out_other = (long long)ld1 * B2; d.out_cnt = B2; d.out_c = B2 / 2;
         d.mode = 2;
         // slabs without support voxels: their rows are skipped by I1 and masked

@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_col_mix(ColPassArg
     const int in_base = Lay::idx(j, vc);
     cplx<T> v[N1][8];
     {
-        const cplx<T> *in = a.in + (long long)other * a.in_other + (long long)col * a.col_stride;
+        const cplx<T> *in = a.in + (long long)other * a.in_other + tile_at(a, tile, a.in_blk) +
+            (long long)c * a.col_stride;
         const unsigned idim = (unsigned)a.in_dim;
 #pragma unroll
         for (int k = 0; k < 8; ++k)
@@ -121,7 +122,8 @@ __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_col_mix(ColPassArg
         reg_fft<T, N2, Lay, true, N1>(v, sA, sB, buf, j, vc, in_base, twp);
         mix_final<T, N2, N1, true>(v, j, tw);
     }
-    cplx<T> *out = a.out + (long long)other * a.out_other + (long long)col * a.col_stride;
+    cplx<T> *out = a.out + (long long)other * a.out_other + tile_at(a, tile, a.out_blk) +
+        (long long)c * a.col_stride;
     const unsigned odim = (unsigned)a.out_dim;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {

@@ -489,6 +489,9 @@ template <typename T> struct ColPassArgs {
     int W, P;
     int ncols;
     long long col_stride;
+    // Columns in blocks of W << blk (see tile_at); 0: evenly spaced
+    long long in_blk, out_blk;
+    int blk;
     const cplx<T> *in;
     long long in_dim, in_other;
     int in_cnt, in_c;
@@ -545,6 +548,15 @@ __device__ __forceinline__ void capture_rfree(const cplx<T> *s, const ColPassArg
     }
 }
 
+// offset of a tile's first column: blk_stride (in_blk or out_blk) elements lie
+// between blocks of 2^blk tiles, and the columns of a block are evenly spaced
+template <typename T>
+__device__ __forceinline__ long long tile_at(const ColPassArgs<T> &a, int tile, long long blk_stride)
+{
+    const int sub = tile & ((1 << a.blk) - 1);
+    return (long long)(tile >> a.blk) * blk_stride + (long long)(sub * a.W) * a.col_stride;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kTileMaxThreads<T>) k_colpass(ColPassArgs<T> a)
 {
@@ -559,19 +571,19 @@ __global__ void __launch_bounds__(kTileMaxThreads<T>) k_colpass(ColPassArgs<T> a
 
     for (int i = tid; i < n * P; i += nt) s[i] = zero;
     __syncthreads();
-    const cplx<T> *in = a.in + (long long)other * a.in_other;
+    const cplx<T> *in = a.in + (long long)other * a.in_other + tile_at(a, tile, a.in_blk);
     if (a.col_stride == 1) {
         for (int idx = tid; idx < a.in_cnt * W; idx += nt) {
             const int e = idx / W, c = idx - e * W;
             const int col = tile * W + c;
-            if (col < a.ncols) s[wrap(e - a.in_c, n) * P + c] = in[(long long)col + (long long)e * a.in_dim];
+            if (col < a.ncols) s[wrap(e - a.in_c, n) * P + c] = in[c + (long long)e * a.in_dim];
         }
     } else {
         for (int idx = tid; idx < a.in_cnt * W; idx += nt) {
             const int c = idx / a.in_cnt, e = idx - c * a.in_cnt;
             const int col = tile * W + c;
             if (col < a.ncols)
-                s[wrap(e - a.in_c, n) * P + c] = in[(long long)col * a.col_stride + (long long)e * a.in_dim];
+                s[wrap(e - a.in_c, n) * P + c] = in[(long long)c * a.col_stride + (long long)e * a.in_dim];
         }
     }
     __syncthreads();
@@ -621,14 +633,14 @@ __global__ void __launch_bounds__(kTileMaxThreads<T>) k_colpass(ColPassArgs<T> a
         __syncthreads();
     }
     if (a.mode & 2) fft_tile<T>(s, a.pl, W, P, a.tw, true);
-    cplx<T> *out = a.out + (long long)other * a.out_other;
+    cplx<T> *out = a.out + (long long)other * a.out_other + tile_at(a, tile, a.out_blk);
     if (a.col_stride == 1) {
         for (int idx = tid; idx < a.out_cnt * W; idx += nt) {
             const int e = idx / W, c = idx - e * W;
             const int col = tile * W + c;
             if (col < a.ncols) {
                 cplx<T> v = s[wrap(e - a.out_c, n) * P + c];
-                out[(long long)col + (long long)e * a.out_dim] = mk(v.x * a.scale, v.y * a.scale);
+                out[c + (long long)e * a.out_dim] = mk(v.x * a.scale, v.y * a.scale);
             }
         }
     } else {
@@ -637,7 +649,7 @@ __global__ void __launch_bounds__(kTileMaxThreads<T>) k_colpass(ColPassArgs<T> a
             const int col = tile * W + c;
             if (col < a.ncols) {
                 cplx<T> v = s[wrap(e - a.out_c, n) * P + c];
-                out[(long long)col * a.col_stride + (long long)e * a.out_dim] = mk(v.x * a.scale, v.y * a.scale);
+                out[(long long)c * a.col_stride + (long long)e * a.out_dim] = mk(v.x * a.scale, v.y * a.scale);
             }
         }
     }

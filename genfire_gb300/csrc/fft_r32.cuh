@@ -22,8 +22,6 @@
 
 #include "fft_reg.cuh"
 
-#include <cuda.h>  // CUtensorMap (the type only; the map is encoded by the host)
-
 namespace gf {
 
 template <int N> struct R32 {
@@ -284,7 +282,8 @@ __device__ __forceinline__ void col_r32_tile(const ColPassArgs<T> &a, cplx<T> *s
         fwd_layout = true;
     }
     if (!fwd_layout || !cv) return;
-    cplx<T> *out = a.out + (long long)other * a.out_other + (long long)col * a.col_stride;
+    cplx<T> *out = a.out + (long long)other * a.out_other + tile_at(a, tile, a.out_blk) +
+        (long long)c * a.col_stride;
     const unsigned odim = (unsigned)a.out_dim;
 #pragma unroll
     for (int sl = 0; sl < 32; ++sl) {
@@ -320,7 +319,8 @@ __global__ void __launch_bounds__(R32<N>::THREADS, r32_col_min_blocks(N)) k_col_
     if (a.zmask && !a.zmask[other]) {
         // a slab without support voxels (see ColPassArgs::zmask)
         if (a.zmask_zero && cv) {
-            cplx<T> *out = a.out + (long long)other * a.out_other + (long long)col * a.col_stride;
+            cplx<T> *out = a.out + (long long)other * a.out_other + tile_at(a, tile, a.out_blk) +
+                (long long)c * a.col_stride;
 #pragma unroll 4
             for (int m = 0; m < 32; ++m) {
                 int e = t + P * m + a.out_c;
@@ -340,13 +340,14 @@ __global__ void __launch_bounds__(R32<N>::THREADS, r32_col_min_blocks(N)) k_col_
         const long long fb = (long long)blockIdx.y * gridDim.x + blockIdx.x + r32_prefetch_ahead(N, ZIN && ZOUT);
         if (fb < nb && a.col_stride == 1 && a.in_dim < kR32PrefetchSpan) {
             const int ftile = (int)(fb % gridDim.x), fother = (int)(fb / gridDim.x);
-            const cplx<T> *fin = a.in + (long long)fother * a.in_other + (long long)ftile * W;
+            const cplx<T> *fin = a.in + (long long)fother * a.in_other + tile_at(a, ftile, a.in_blk);
             for (int r = threadIdx.x; r < a.in_cnt; r += G::THREADS)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(fin + (long long)r * a.in_dim));
         }
     }
     {
-        const cplx<T> *in = a.in + (long long)other * a.in_other + (long long)col * a.col_stride;
+        const cplx<T> *in = a.in + (long long)other * a.in_other + tile_at(a, tile, a.in_blk) +
+            (long long)c * a.col_stride;
         const unsigned idim = (unsigned)a.in_dim;
 #pragma unroll
         for (int m = 0; m < 32; ++m) {
@@ -369,10 +370,8 @@ __global__ void __launch_bounds__(R32<N>::THREADS, r32_col_min_blocks(N)) k_col_
 // Persistent fused 512-point complex64 pass (F3 at 512 points): CTAs loop over
 // the tiles (tile, other) = (item % tiles_x, item / tiles_x), item += gridDim.x,
 // and each tile's input (the centred half of the box: N/2 rows x W columns,
-// 16 KB) comes into a shared-memory stage by a TMA tensor copy issued one tile
-// ahead, while the CTA transforms the current one.  tmap describes the input
-// as floats: {2 x in_other, in_dim / in_other, in_cnt} with the box
-// {2 W, 1, N/2} (x = 2 W tile, 64-byte aligned).  The wait for a copy is bounded
+// 16 KB in one piece) comes into a shared-memory stage by a bulk copy issued one
+// tile ahead, while the CTA transforms the current one.  The wait for a copy is bounded
 // (clock64); on expiry the CTA stops at a reducing barrier, sets *a.err, waits
 // (full limit) for the copy in flight and returns.
 namespace r32tma {
@@ -397,14 +396,12 @@ __device__ __forceinline__ bool wait(uint64_t *bar, uint32_t parity)
         if (clock64() - t0 > kWaitCycles) return false;
     return true;
 }
-__device__ __forceinline__ void load_tile(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar, uint32_t bytes)
+__device__ __forceinline__ void load_tile(void *dst, const void *src, uint64_t *bar, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(bar)), "r"(bytes) : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            saddr(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(0), "r"(saddr(bar))
-        : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(saddr(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(saddr(bar))
+                 : "memory");
 }
 }  // namespace r32tma
 
@@ -414,7 +411,7 @@ template <int N> constexpr size_t r32_tma_smem() { return r32_tma_stage_offset<N
 
 template <int N>
 __global__ void __launch_bounds__(R32<N>::THREADS, 4)
-    k_col_r32_tma(ColPassArgs<float> a, const __grid_constant__ CUtensorMap tmap, int tiles_x, int ntiles)
+    k_col_r32_tma(ColPassArgs<float> a, int tiles_x, int ntiles)
 {
     pass_begin();
     using G = R32<N>;
@@ -430,9 +427,12 @@ __global__ void __launch_bounds__(R32<N>::THREADS, 4)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    auto fetch = [&](int i) {
+        const float2 *src = a.in + (long long)(i / tiles_x) * a.in_other + tile_at(a, i % tiles_x, a.in_blk);
+        r32tma::load_tile(stage, src, bar, kBytes);
+    };
     int item = blockIdx.x;
-    if (threadIdx.x == 0 && item < ntiles)
-        r32tma::load_tile(stage, &tmap, 2 * W * (item % tiles_x), item / tiles_x, bar, kBytes);
+    if (threadIdx.x == 0 && item < ntiles) fetch(item);
     bool pending = item < ntiles;  // a copy is in flight (uniform)
     uint32_t phase = 0;
     bool ok = true;
@@ -450,13 +450,13 @@ __global__ void __launch_bounds__(R32<N>::THREADS, 4)
             if (m >= 8 && m < 24) x[m] = mk(0.f, 0.f);
             else x[m] = stage[(t + G::half_off(m)) * W + c];
         }
-        // generic-proxy reads of the stage before the next tensor copy (async proxy)
+        // generic-proxy reads of the stage before the next copy (async proxy)
         // overwrites it; after the barrier the stage and the exchange buffer are free
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         const int next = item + gridDim.x;
         if (next < ntiles) {
-            if (threadIdx.x == 0) r32tma::load_tile(stage, &tmap, 2 * W * (next % tiles_x), next / tiles_x, bar, kBytes);
+            if (threadIdx.x == 0) fetch(next);
             pending = true;
         }
         col_r32_tile<float, N, true, true>(a, s, x, item % tiles_x, item / tiles_x, tiles_x);

@@ -432,7 +432,8 @@ __global__ void __launch_bounds__(col_threads<T, N, NC>(), kRegMinBlocks<T>) k_c
     const int in_base = Lay::idx(j, c);
     cplx<T> v[NC][8];
     {
-        const cplx<T> *in = a.in + (long long)other * a.in_other + (long long)col * a.col_stride;
+        const cplx<T> *in = a.in + (long long)other * a.in_other + tile_at(a, tile, a.in_blk) +
+            (long long)c * a.col_stride;
         const unsigned idim = (unsigned)a.in_dim;
         int e = j + a.in_c;
         if (e >= N) e -= N;
@@ -466,7 +467,8 @@ __global__ void __launch_bounds__(col_threads<T, N, NC>(), kRegMinBlocks<T>) k_c
         }
         reg_fft<T, N, Lay, true, NC>(v, sA, sB, buf, j, c, in_base, twp);
     }
-    cplx<T> *out = a.out + (long long)other * a.out_other + (long long)col * a.col_stride;
+    cplx<T> *out = a.out + (long long)other * a.out_other + tile_at(a, tile, a.out_blk) +
+        (long long)c * a.col_stride;
     const unsigned odim = (unsigned)a.out_dim;
     {
         constexpr int R = P2Plan<N>::radix(NST - 1);

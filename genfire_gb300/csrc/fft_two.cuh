@@ -291,7 +291,8 @@ __device__ __noinline__ void two_transform(const ColPassArgs<T> &a, const Plan &
             for (int m = 0; m < R; ++m) x[m] = s[((tA + tp.R2 * m) << lw) + c];
             __syncthreads();  // the natural-order tile is read before the exchange overwrites it
         } else {
-            const cplx<T> *in = a.in + (long long)other * a.in_other + (long long)col * a.col_stride;
+            const cplx<T> *in = a.in + (long long)other * a.in_other + tile_at(a, (int)blockIdx.x, a.in_blk) +
+                (long long)c * a.col_stride;
             const unsigned idim = (unsigned)a.in_dim;
             int e = tA + a.in_c;
             if (e >= N) e -= N;
@@ -319,7 +320,8 @@ __device__ __noinline__ void two_transform(const ColPassArgs<T> &a, const Plan &
         // element k = t + R1 k2, an inverse's at (N - k) mod N
         const int step = dir ? -tp.R1 : tp.R1;
         if (last) {
-            cplx<T> *out = a.out + (long long)other * a.out_other + (long long)col * a.col_stride;
+            cplx<T> *out = a.out + (long long)other * a.out_other + tile_at(a, (int)blockIdx.x, a.out_blk) +
+                (long long)c * a.col_stride;
             const unsigned odim = (unsigned)a.out_dim;
             int e = (dir && tB ? N - tB : tB) + a.out_c;
             if (e >= N) e -= N;
