@@ -28,6 +28,7 @@
 #include "internal.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -1740,6 +1741,51 @@ void recon_destroy(genfire_recon *r)
 // batches: one graph holds one iteration of every member problem as
 // independent child graphs, so one launch runs them all concurrently
 // ===========================================================================
+// The branch (0 .. S - 1) of each member, given its grid points in descending
+// order.  A pass over kFullGrid points has more CTAs than the chip holds at
+// once.  Members from there on share two branches, each going to the one with
+// less before it: the next kernel of the other branch fills the chip while a
+// pass ends, and the working sets of two 256^3 grids still share the L2, those
+// of more do not.  A third branch where two would leave one of them idle for
+// long.  The smaller members, a launch latency per pass, slow the large ones
+// down when they run beside them, so they get as few branches as it takes to be
+// done by the time the large ones are; with no large member, all of them.
+// ms per iteration, members dealt to 8 branches in turn -> this:
+//   objects of 192, 160, 128, 2 x 96, 2 x 64, 48   0.751 -> 0.675
+//   6 x 128, 2 x 96                                0.472 -> 0.411
+//   160, 128, 96, 48                               0.328 -> 0.293
+//   3 x 160 (two branches 0.514)                   0.505 -> 0.505
+//   8 x 64 (one branch 0.185)                      the same, 0.08
+static std::vector<int> batch_branches(const std::vector<double> &points, int S)
+{
+    constexpr double kFullGrid = 6e6;
+    constexpr double kLargeUs = 5e-6, kSmallUs = 25;  // an iteration: per point of a large grid, of a small one
+    const int count = (int)points.size();
+    int large = 0;
+    double sum = 0;
+    while (large < count && points[large] >= kFullGrid) sum += points[large++];
+    std::vector<int> branch(count);
+    // members from..to on the branches b0 .. b0 + nb - 1; returns the longest branch's points
+    auto deal = [&](int from, int to, int b0, int nb) {
+        std::vector<double> load(nb, 0.0);
+        for (int i = from; i < to; ++i) {
+            const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+            load[k] += points[i];
+            branch[i] = b0 + k;
+        }
+        return *std::max_element(load.begin(), load.end());
+    };
+    int nb = std::min(large, std::min(S, 2));
+    if (nb && deal(0, large, 0, nb) * nb > 1.25 * sum && std::min(large, S) > nb) deal(0, large, 0, ++nb);
+    if (large < count) {
+        int ns = S - nb;
+        if (large) ns = std::min(ns, std::max(1, (int)std::ceil(kSmallUs * (count - large) / (kLargeUs * sum))));
+        if (ns > 0) deal(large, count, nb, ns);
+        else deal(large, count, 0, S);
+    }
+    return branch;
+}
+
 genfire_recon_batch *recon_batch_create(genfire_ctx *ctx, genfire_recon *const *members, int count)
 {
     if (count < 1) fail(GENFIRE_ERR_ARG, "batch: at least one reconstruction.");
@@ -1750,9 +1796,8 @@ genfire_recon_batch *recon_batch_create(genfire_ctx *ctx, genfire_recon *const *
             if (members[j] == members[i]) fail(GENFIRE_ERR_ARG, "batch: a reconstruction appears twice.");
     }
     // One graph of one iteration of every member: a fork/join capture in which
-    // the members' launches go to up to 8 branch streams (largest grids first,
-    // dealt round-robin), so the graph holds parallel chains of kernels and small
-    // members run beside the large ones.
+    // the members' launches go to up to 8 branch streams (batch_branches), so the
+    // graph holds parallel chains of kernels.
     auto *b = new genfire_recon_batch();
     b->ctx = ctx;
     b->members.assign(members, members + count);
@@ -1774,13 +1819,16 @@ genfire_recon_batch *recon_batch_create(genfire_ctx *ctx, genfire_recon *const *
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
             return members[x]->impl->grid_points() > members[y]->impl->grid_points();
         });
+        std::vector<double> points;
+        for (int n = 0; n < count; ++n) points.push_back((double)members[order[n]]->impl->grid_points());
+        const std::vector<int> branch = batch_branches(points, S);
         for (int i = 0; i < count; ++i) members[i]->impl->prepare_capture();
         cudaStream_t st = ctx->stream;
         GF_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         try {
             GF_CUDA(cudaEventRecord(b->events[S], st));  // fork
             for (int k = 0; k < S; ++k) GF_CUDA(cudaStreamWaitEvent(b->branches[k], b->events[S], 0));
-            for (int n = 0; n < count; ++n) members[order[n]]->impl->enqueue(b->branches[n % S]);
+            for (int n = 0; n < count; ++n) members[order[n]]->impl->enqueue(b->branches[branch[n]]);
             for (int k = 0; k < S; ++k) {  // join
                 GF_CUDA(cudaEventRecord(b->events[k], b->branches[k]));
                 GF_CUDA(cudaStreamWaitEvent(st, b->events[k], 0));
