@@ -420,7 +420,8 @@ def run_ours(args, ws, rank, local, pg):
         "fft_pass_variants": {"F2": tuned[0], "F3": tuned[1], "I2": tuned[2],
                               "legend": "autotuned at setup: 0 generic shared-memory engine, 1 radix-8 register "
                                         "engine one column per thread, 2 the same with two columns per thread, "
-                                        "3 mixed-radix engine, 4 radix-32 engine (512 or 1024 points, one exchange)"},
+                                        "3 mixed-radix engine, 4 radix-32 engine (128 to 1024 points, one exchange), "
+                                        "5 the same fed by bulk copies, 6 two register stages"},
         "cpu_baseline": cpu,
         "clocks": clk,
         "gpu_launches": len(ms) * K,
@@ -443,7 +444,8 @@ def gridding_roofline(flops, nk, D, stages, tile=128):
         peak, kind = 1900.0, "fallback"
     ms = stages["dft_kernel"]
     tiles = float(np.sum(np.ceil(np.asarray(nk, dtype=np.float64) / tile)))
-    k_pad, n_pad = -(-D // 32) * 32, -(-D // 16) * 16
+    rows = D // 2 if tile == 128 else D  # the default form multiplies the projection folded over its rows
+    k_pad, n_pad = -(-rows // 32) * 32, -(-D // 16) * 16
     executed = tiles * tile * k_pad * n_pad * 2.0 * 6
     ach = flops / (ms * 1e-3) / 1e12
     return {"kernel": "k_dft_tcgen05" if tile == 128 else "k_dft_tcgen05_w", "bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
@@ -451,7 +453,7 @@ def gridding_roofline(flops, nk, D, stages, tile=128):
             "executed_tflops": executed / (ms * 1e-3) / 1e12, "executed_frac": executed / (ms * 1e-3) / 1e12 / peak,
             "note": "achieved counts the useful DFT flops; executed counts the split products the tensor cores "
                     "run (3 per complex-real product, Re and Im: 6 products of 2 flops per MAC, on whole tiles "
-                    "and the projection padded to 32 rows and 16 columns)"}
+                    "and the projection, in the default form folded to half its rows, padded to 32 rows and 16 columns)"}
 
 
 def projector_leg(G, ctx, vol, w, reps=5):
@@ -534,7 +536,7 @@ def batch_leg(G, ctx, K, quick):
             "batched_problem_iters_per_s": n * K / t_batch, "sequential_problem_iters_per_s": n * K / t_seq,
             "batched_over_sequential": t_seq / t_batch, "batched_ms": t_batch * 1e3, "sequential_ms": t_seq * 1e3,
             "note": "wall time with a stream synchronize at the end of each leg; one graph launch per batched "
-                    "iteration runs every problem's iteration as an independent child graph"}
+                    "iteration runs every problem's iteration in parallel chains of kernels"}
 
 
 def cpu_baseline(w, d_M64):

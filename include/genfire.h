@@ -225,7 +225,7 @@ genfire_status genfire_recon_destroy(genfire_recon *r);
 
 /* Batches of independent reconstructions (problems of different sizes,
  * precisions and projection counts) iterated together: one CUDA graph holds
- * one iteration of every member as independent child graphs, so each launch
+ * one iteration of every member in parallel chains of kernels, so each launch
  * runs all members' iterations concurrently on the device.  No counterpart in
  * the reference, which reconstructs one object per call.  Every member must
  * have been created on ctx; the batch does not own them: destroy the batch
@@ -251,8 +251,10 @@ genfire_status genfire_recon_batch_destroy(genfire_recon_batch *b);
  * the dim-2 forward, the fused dim-3 and the dim-2 inverse pass; 0 = generic
  * shared-memory engine, 1 = register-resident radix 8, one column per thread,
  * 2 = the same with two columns per thread, 3 = mixed radix (3 or 5 times a
- * power of two), 4 = radix 32 x 16 or 32 x 32 for 512 or 1024 complex64
- * points (one shared-memory exchange per transform), -1 = built-in choice.
+ * power of two), 4 = radix 32 for 128 to 1024 complex64 points (one
+ * shared-memory exchange per transform), 5 = the same for the fused 512-point
+ * pass, fed by bulk copies, 6 = two register stages of up to 32 points each
+ * (any other length that splits so), -1 = built-in choice.
  * GENFIRE_COL_VARIANT=<v>
  * forces variant v wherever it is valid. */
 genfire_status genfire_recon_tuning(genfire_recon *r, int32_t *variants);
