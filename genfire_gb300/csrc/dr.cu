@@ -413,6 +413,10 @@ template <typename T> static int autotune_colpass(ColPassArgs<T> a, int other, c
     float best_ms = 0, default_ms = -1;
     for (int v : {kColGeneric, kColReg1, kColReg2, kColMix, kColR32, kColR32Tma, kColTwo}) {
         if (!col_variant_ok(a, v)) continue;
+        // lengths whose engine is the two-stage one: the generic engine is near it
+        // only where a pass is one launch latency long, and choosing between them
+        // by time would give two processes different bits
+        if (v == kColGeneric && default_col_variant(a) == kColTwo) continue;
         launch_colpass<T>(a, other, st, v);
         GF_CUDA(cudaEventRecord(e0, st));
         for (int r = 0; r < 3; ++r) launch_colpass<T>(a, other, st, v);

@@ -1100,7 +1100,7 @@ template <bool F16> __device__ __forceinline__ void split_to(float x, uint16_t *
 // Grid: x = block, y = K chunk.  The sums are formed in FP64, whose pipe takes 64
 // cycles a warp instruction, so the padding (7/8 of the block of a 32 x 32
 // projection) does none of it.  32 x 32, 13 projections: the DFT's stage 38.6 ->
-// 33.4 us; 256 x 256, 90: the whole gridding call 2.38 -> 2.30 ms
+// 33.4 us; 256 x 256, 90: within 1 % of the call.
 constexpr int kFoldThreads = 1024;  // four elements each: a chunk is one trip to memory long
 template <bool F16>
 __global__ void __launch_bounds__(kFoldThreads) k_fold_split(const double *__restrict__ proj, int D1, int D2, int D2p,
