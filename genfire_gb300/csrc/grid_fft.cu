@@ -77,6 +77,8 @@ struct __align__(16) FftSlice {
 };
 
 constexpr int kGatherThreads = 128;
+constexpr int kMaxCube = 1290;  // the largest m with m^3 below 2^31
+constexpr size_t gather_smem(int m) { return sizeof(double) * 6 * (size_t)(2 * (m / 2) + 1); }
 
 // Conversions between single and double by integer arithmetic, where the
 // hardware's would issue on the FP64 pipe: exact widening, and narrowing rounded
@@ -349,9 +351,8 @@ static void grid_fft_t(genfire_ctx *ctx, const genfire_params &p, const double *
     const double reach = std::min(p.interpolationCutoffDistance, 1.7321 * (g.s + 0.5));
     g.reach = (float)reach + 0.01f;
     const int h = m / 2;
-    const size_t smem = sizeof(double) * 6 * (size_t)(2 * h + 1);
-    GF_CUDA(cudaFuncSetAttribute((const void *)k_fft_gather<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_gather<T><<<dim3(2 * h + 1, h + 1), kGatherThreads, smem, st>>>(
+    raise_smem_limit(ctx->device, (const void *)k_fft_gather<T>, gather_smem(kMaxCube));
+    k_fft_gather<T><<<dim3(2 * h + 1, h + 1), kGatherThreads, gather_smem(m), st>>>(
         X.as<cplx<T>>(), dsl.as<FftSlice>(), g, dpairs.as<unsigned long long>(), reinterpret_cast<cplx<T> *>(d_M));
     GF_CHECK_LAUNCH();
     X.release();
@@ -371,7 +372,8 @@ void grid_fft(genfire_ctx *ctx, const genfire_params &p, const double *d_proj, c
         fail(GENFIRE_ERR_ARG, "FFT gridding: Dim2 * oversamplingRatio (1 + (Dim2-1) * oversamplingRatio for odd "
                               "Dim2) must be an integer.");
     if (m < p.Dim1 || m < p.Dim2) fail(GENFIRE_ERR_ARG, "FFT gridding: the grid is smaller than the projections.");
-    if ((long long)m * m * m >= (1LL << 31)) fail(GENFIRE_ERR_ARG, "FFT gridding: grid too large (m^3 must stay below 2^31).");
+    static_assert((long long)kMaxCube * kMaxCube * kMaxCube < (1LL << 31), "largest cube");
+    if (m > kMaxCube) fail(GENFIRE_ERR_ARG, "FFT gridding: grid too large (m^3 must stay below 2^31).");
     if (p.NumProjs > 65535) fail(GENFIRE_ERR_ARG, "FFT gridding: at most 65535 projections.");
     if (p.precision == GENFIRE_PREC_FP64) grid_fft_t<double>(ctx, p, d_proj, angles, d_M, d_rec, npairs);
     else grid_fft_t<float>(ctx, p, d_proj, angles, d_M, d_rec, npairs);

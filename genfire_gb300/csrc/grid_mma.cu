@@ -1232,8 +1232,7 @@ __global__ void k_fill_f32(float *__restrict__ x, int n, float v)
     if (i < n) x[i] = v;
 }
 
-// The DFT kernels' dynamic shared memory is raised once per device and kernel.
-static void ws_smem_attr(int device, const void *kern, size_t bytes)
+void raise_smem_limit(int device, const void *kern, size_t bytes)
 {
     static std::mutex m;
     static std::set<std::pair<int, const void *>> done;
@@ -1347,7 +1346,7 @@ void dft_tcgen05(genfire_ctx *ctx, const double *d_proj, int D1, int D2, int n1,
         kern = fp16 ? (pow2 ? (const void *)k_dft_tcgen05<true, true> : (const void *)k_dft_tcgen05<true, false>)
                     : (pow2 ? (const void *)k_dft_tcgen05<false, true> : (const void *)k_dft_tcgen05<false, false>);
     const size_t smem = wide ? kWSmem : kWsSmem;
-    ws_smem_attr(ctx->device, kern, smem);
+    raise_smem_limit(ctx->device, kern, smem);
     const int grid = (int)std::min<long long>(nunits, (long long)ctx->sm_count);
     if (ev_begin) GF_CUDA(cudaEventRecord(ev_begin, st));
     void *args[] = {&a};

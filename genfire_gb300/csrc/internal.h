@@ -95,6 +95,12 @@ void dft_tcgen05(genfire_ctx *ctx, const double *d_proj, int D1, int D2, int n1,
                  const std::vector<long long> &nk, const long long *d_off, const float *d_u, const float *d_v,
                  float2 *d_F, int *d_err, cudaEvent_t ev_begin, cudaEvent_t ev_end, bool fp16);
 
+// Raises a kernel's dynamic shared memory limit, once per device and kernel: the
+// limit belongs to the device, not to a context, so it is set to the most that any
+// call can need and never to a call's own size, which another thread could lower
+// before its launch.
+void raise_smem_limit(int device, const void *kern, size_t bytes);
+
 // Selection of one projection into host arrays (test entry point).
 long long select_one(genfire_ctx *ctx, const genfire_params &p, double phi, double theta, double psi,
                      long long cap, int64_t *ind, float *dist, float *u, float *v);
