@@ -393,6 +393,8 @@ static ProjTexture *atlas(genfire_ctx *ctx, int n1, int n2, int n3)
 {
     ProjTexture *&cur = ctx->proj_texture;
     if (cur && cur->t.n1 == n1 && cur->t.n2 == n2 && cur->t.n3 == n3) return cur;
+    // a slice fits the sides, and the slices are the writing kernel's z blocks
+    if (n1 > kAtlasSide || n2 > kAtlasSide || n3 > 65535) return nullptr;
     int lgx = 0;  // the fewest slices across that keep the height in bounds
     while ((long long)n2 * cdiv(n3, 1 << lgx) > kAtlasSide) ++lgx;
     const size_t w = (size_t)n1 << lgx, h = (size_t)n2 * cdiv(n3, 1 << lgx);
