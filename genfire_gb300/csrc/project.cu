@@ -201,14 +201,16 @@ struct ProjAtlas {
     int n1, n2, n3, lgx;
 };
 
-// grid: x over dim 1, y = dim 2, z = slice
+// grid: x over the pixels of a slice, y = slice.  (With a row per y, a volume of 2 x
+// 4096 x 2048 left 254 of 256 threads idle: 4.7 ms a call, 0.46 here.)
 __global__ void __launch_bounds__(256) k_atlas_write(const float *__restrict__ vol, long long vs1, long long vs2,
                                                      ProjAtlas t, cudaSurfaceObject_t surf)
 {
-    const int j = blockIdx.y, k = blockIdx.z;
+    const int px = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+    if (px >= t.n1 * t.n2) return;
+    const int j = px / t.n1, i = px - j * t.n1;
     const int x0 = (k & ((1 << t.lgx) - 1)) * t.n1, y = (k >> t.lgx) * t.n2 + j;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.n1; i += gridDim.x * blockDim.x)
-        surf2Dwrite(vol[i + vs1 * j + vs2 * k], surf, (x0 + i) * (int)sizeof(float), y);
+    surf2Dwrite(vol[i + vs1 * j + vs2 * k], surf, (x0 + i) * (int)sizeof(float), y);
 }
 
 // small non-negative integer to float without a conversion instruction
@@ -393,7 +395,7 @@ static ProjTexture *atlas(genfire_ctx *ctx, int n1, int n2, int n3)
 {
     ProjTexture *&cur = ctx->proj_texture;
     if (cur && cur->t.n1 == n1 && cur->t.n2 == n2 && cur->t.n3 == n3) return cur;
-    // a slice fits the sides, and the slices are the writing kernel's z blocks
+    // a slice fits the sides, and the slices are the writing kernel's y blocks
     if (n1 > kAtlasSide || n2 > kAtlasSide || n3 > 65535) return nullptr;
     int lgx = 0;  // the fewest slices across that keep the height in bounds
     while ((long long)n2 * cdiv(n3, 1 << lgx) > kAtlasSide) ++lgx;
@@ -445,7 +447,7 @@ static void project_t(genfire_ctx *ctx, const T *vol, int n1, int n2, int n3, lo
     dim3 grid(nblk, P);
     if (at) {
         if constexpr (sizeof(T) == 4) {
-            k_atlas_write<<<dim3(cdiv(n1, 256), n2, n3), 256, 0, st>>>(vol, vs1, vs2, at->t, at->surf);
+            k_atlas_write<<<dim3(cdiv(npix, 256), n3), 256, 0, st>>>(vol, vs1, vs2, at->t, at->surf);
             GF_CHECK_LAUNCH();
             k_project_tex<<<grid, kProjThreads, 0, st>>>(at->tex, at->t, d_R, d_proj, d_meas, part.as<double>());
         }

@@ -34,3 +34,21 @@ def test_sides_beyond_the_texture(lib, ctx, shape):
     for q in range(0, P, 5):
         one = ctx.project(vol, angles[q:q + 1], precision=lib.PREC_MIXED)
         assert np.abs(got[:, :, q] - one[:, :, 0]).max() <= 1e-6 * max(np.abs(one).max(), 1)
+
+
+def test_thin_volumes_take_no_longer(lib, ctx):
+    """The same number of samples in slices of 2 x 4096 and of 2048 x 4 pixels; two
+    threads of 256 at work made it ten times the time."""
+    import time
+    rng = np.random.default_rng(3)
+    angles = np.asfortranarray([(30., 40., 50.)])
+    best = []
+    for shape in ((2, 4096, 2048), (2048, 4, 2048)):
+        vol = np.asfortranarray(rng.random(shape).astype(np.float32))
+        t = []
+        for _ in range(8):
+            t0 = time.perf_counter()
+            ctx.project(vol, angles, precision=lib.PREC_MIXED)
+            t.append(time.perf_counter() - t0)
+        best.append(min(t))
+    assert best[0] < 4 * best[1], best
