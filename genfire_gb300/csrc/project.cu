@@ -241,13 +241,17 @@ __global__ void __launch_bounds__(kProjThreads)
         const float h1 = (float)(n1 - 2), h2 = (float)(n2 - 2), h3 = (float)(n3 - 2);
         const float f1 = (float)n1, f2 = (float)n2;
         const int mask = (1 << t.lgx) - 1;
-        // the samples that can lie in the volume: b + Z r within [0, e] for each
-        // coordinate, a sample wider on either side than the rounded bounds
+        // the samples that can lie in the volume: b + Z r within [0, e'] for each
+        // coordinate, a sample wider on either side than the rounded bounds.  e' is
+        // a unit in the last place or two beyond e: the loop tests the rounded
+        // coordinate, and what lies within half a unit above e rounds onto it, which
+        // at a slope of 1e-6 is a stretch of 8 samples at 256 points (at 0 the sign
+        // is exact).
         float zlo = (float)(-c3), zhi = (float)(n3 - 1 - c3);
         auto clip = [&](float b, float r, float e) {
             if (fabsf(r) < 1e-6f) return;  // (Z r stays below 0.04: the test in the loop decides)
             const float inv = 1.f / r;
-            float u = -b * inv, v = (e - b) * inv;
+            float u = -b * inv, v = (fmaf(e, 0x1p-23f, e) - b) * inv;
             if (u > v) { const float q = u; u = v; v = q; }
             zlo = fmaxf(zlo, u);
             zhi = fminf(zhi, v);
@@ -255,7 +259,9 @@ __global__ void __launch_bounds__(kProjThreads)
         clip(bx, r6, e1);
         clip(by, r7, e2);
         clip(bz, r8, e3);
-        const int k0 = max(0, (int)floorf(zlo) + c3 - 1), k1 = min(n3 - 1, (int)ceilf(zhi) + c3 + 1);
+        // (a line that misses the volume may have its bounds anywhere)
+        const int k0 = max(0, (int)floorf(fminf(zlo, (float)n3)) + c3 - 1);
+        const int k1 = min(n3 - 1, (int)ceilf(fmaxf(zhi, -(float)n3)) + c3 + 1);
         float part_acc = 0.f;
         auto sample = [&](int k) -> float {
             const float Z = (float)(k - c3);
