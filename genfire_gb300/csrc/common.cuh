@@ -62,6 +62,11 @@ struct Error {
 // ---------------------------------------------------------------------------
 // device buffers (stream-ordered allocation on the context stream)
 // ---------------------------------------------------------------------------
+
+// Frees what the contexts keep on the current device for their next calls and no
+// call is using (project.cu); true when that was anything.
+bool release_kept_memory();
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -73,7 +78,19 @@ struct DevBuf {
         release();
         s = st;
         bytes = n;
-        if (n) GF_CUDA(cudaMallocAsync(&p, n, st));
+        if (!n) return;
+        cudaError_t e = cudaMallocAsync(&p, n, st);
+        if (e == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();  // the failure must not surface at a later launch's check
+            if (release_kept_memory()) e = cudaMallocAsync(&p, n, st);
+            if (e == cudaErrorMemoryAllocation) {
+                (void)cudaGetLastError();
+                p = nullptr;
+                bytes = 0;
+                throw Error{GENFIRE_ERR_OOM, "GENFIRE: device memory exhausted: " + std::to_string(n) + " bytes wanted"};
+            }
+        }
+        GF_CUDA(e);
     }
     void release()
     {

@@ -11,8 +11,10 @@
 // and reduced with warp shuffles, per projection, in a fixed order.
 #include "internal.h"
 
-#include <map>
+#include <algorithm>
+#include <memory>
 #include <mutex>
+#include <set>
 
 namespace gf {
 
@@ -372,90 +374,173 @@ __global__ void k_project_sums(const double *__restrict__ part, int nblk, double
 }
 
 // ---------------------------------------------------------------------------
-// The context's atlas: one array, kept for the next call of the same volume
-// size (a series of projector calls, the R-factor monitor) and freed for another
-// size and with the context.  At most kAtlasMax bytes; larger volumes, and
-// sizes whose slices do not fit a 2-D array, keep the load kernel.
+// The context's atlas: one array, kept for the next calls (a series of projector
+// calls, the R-factor monitor), whatever their volumes' sizes as long as they fit
+// it; one that does not fit replaces it by one that holds both.  At most kAtlasMax
+// bytes; larger volumes, and sizes whose slices do not fit a 2-D array, keep the
+// load kernel.  It is freed with the context, and by any call on the device whose
+// allocation fails (release_kept_memory) while no call is using it.
 // ---------------------------------------------------------------------------
 constexpr size_t kAtlasMax = 1u << 30;
 constexpr long long kTexSamples = 1LL << 22;
 constexpr int kAtlasSide = 32768;
 
 struct ProjTexture {
-    ProjAtlas t{0, 0, 0, 0};
+    int device = 0;
+    size_t w = 0, h = 0;  // the array's texels
     cudaArray_t array = nullptr;
     cudaTextureObject_t tex = 0;
     cudaSurfaceObject_t surf = 0;
-    ~ProjTexture()
+    cudaEvent_t used = nullptr;  // after the last launch that reads it
+    bool busy = false;           // a call has taken it and not yet recorded `used`
+    void drop()
     {
         if (tex) cudaDestroyTextureObject(tex);
         if (surf) cudaDestroySurfaceObject(surf);
         if (array) cudaFreeArray(array);
+        tex = 0;
+        surf = 0;
+        array = nullptr;
+        w = h = 0;
     }
-};
-void proj_texture_destroy(ProjTexture *t) { delete t; }
-
-// The context's atlas for a volume size, nullptr when there is none (the size
-// does not qualify or the device has no room).
-static ProjTexture *atlas(genfire_ctx *ctx, int n1, int n2, int n3)
-{
-    ProjTexture *&cur = ctx->proj_texture;
-    if (cur && cur->t.n1 == n1 && cur->t.n2 == n2 && cur->t.n3 == n3) return cur;
-    // a slice fits the sides, and the slices are the writing kernel's y blocks
-    if (n1 > kAtlasSide || n2 > kAtlasSide || n3 > 65535) return nullptr;
-    int lgx = 0;  // the fewest slices across that keep the height in bounds
-    while ((long long)n2 * cdiv(n3, 1 << lgx) > kAtlasSide) ++lgx;
-    const size_t w = (size_t)n1 << lgx, h = (size_t)n2 * cdiv(n3, 1 << lgx);
-    if (w > (size_t)kAtlasSide || w * h * sizeof(float) > kAtlasMax) return nullptr;
-    GF_CUDA(cudaStreamSynchronize(ctx->stream));  // the old one may still be read
-    delete cur;
-    cur = nullptr;
-    auto *a = new ProjTexture();
-    const cudaChannelFormatDesc ch = cudaCreateChannelDesc<float>();
-    cudaError_t e = cudaMallocArray(&a->array, &ch, w, h, cudaArraySurfaceLoadStore | cudaArrayTextureGather);
-    if (e == cudaSuccess) {
+    cudaError_t make(size_t width, size_t height)
+    {
+        const cudaChannelFormatDesc ch = cudaCreateChannelDesc<float>();
+        cudaError_t e = cudaMallocArray(&array, &ch, width, height, cudaArraySurfaceLoadStore | cudaArrayTextureGather);
+        if (e != cudaSuccess) return e;
         cudaResourceDesc rd{};
         rd.resType = cudaResourceTypeArray;
-        rd.res.array.array = a->array;
+        rd.res.array.array = array;
         cudaTextureDesc td{};
         td.addressMode[0] = td.addressMode[1] = cudaAddressModeClamp;
         td.filterMode = cudaFilterModePoint;
         td.readMode = cudaReadModeElementType;
-        e = cudaCreateTextureObject(&a->tex, &rd, &td, nullptr);
-        if (e == cudaSuccess) e = cudaCreateSurfaceObject(&a->surf, &rd);
+        e = cudaCreateTextureObject(&tex, &rd, &td, nullptr);
+        if (e == cudaSuccess) e = cudaCreateSurfaceObject(&surf, &rd);
+        w = width;
+        h = height;
+        return e;
     }
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        delete a;
-        return nullptr;
-    }
-    a->t = ProjAtlas{n1, n2, n3, lgx};
-    cur = a;
-    return a;
+};
+
+// every context's atlas; the lock covers their arrays and flags
+static std::mutex &kept_lock()
+{
+    static std::mutex m;
+    return m;
 }
+static std::set<ProjTexture *> &kept()
+{
+    static std::set<ProjTexture *> s;
+    return s;
+}
+
+void proj_texture_destroy(ProjTexture *t)
+{
+    if (!t) return;
+    std::lock_guard<std::mutex> g(kept_lock());
+    kept().erase(t);
+    t->drop();
+    if (t->used) cudaEventDestroy(t->used);
+    delete t;
+}
+
+bool release_kept_memory()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> g(kept_lock());
+    bool any = false;
+    for (ProjTexture *t : kept())
+        if (t->array && !t->busy && t->device == dev && cudaEventSynchronize(t->used) == cudaSuccess) {
+            t->drop();
+            any = true;
+        }
+    return any;
+}
+
+// A call's use of its context's atlas: t is nullptr when there is none (the
+// volume's size does not qualify or the device has no room).
+struct AtlasUse {
+    ProjTexture *t = nullptr;
+    ProjAtlas lay{0, 0, 0, 0};
+    cudaStream_t st = nullptr;
+    AtlasUse() = default;
+    AtlasUse(const AtlasUse &) = delete;
+    AtlasUse &operator=(const AtlasUse &) = delete;
+    void take(genfire_ctx *ctx, int n1, int n2, int n3, cudaStream_t stream)
+    {
+        // a slice fits the sides, and the slices are the writing kernel's y blocks
+        if (n1 > kAtlasSide || n2 > kAtlasSide || n3 > 65535) return;
+        // the fewest slices across that keep the height within rows
+        auto across = [&](long long rows) {
+            int lgx = 0;
+            while ((1 << lgx) < n3 && (long long)n2 * cdiv(n3, 1 << lgx) > rows) ++lgx;
+            return lgx;
+        };
+        const int lgx = across(kAtlasSide);
+        size_t w = (size_t)n1 << lgx, h = (size_t)n2 * cdiv(n3, 1 << lgx);
+        if (w > (size_t)kAtlasSide || w * h * sizeof(float) > kAtlasMax) return;
+        std::lock_guard<std::mutex> g(kept_lock());
+        ProjTexture *&a = ctx->proj_texture;
+        if (!a) {
+            std::unique_ptr<ProjTexture> n(new ProjTexture());
+            n->device = ctx->device;
+            GF_CUDA(cudaEventCreateWithFlags(&n->used, cudaEventDisableTiming));
+            kept().insert(n.get());
+            a = n.release();
+        }
+        lay = ProjAtlas{n1, n2, n3, across((long long)a->h)};
+        if (!a->array || (size_t)n2 * cdiv(n3, 1 << lay.lgx) > a->h || (size_t)n1 << lay.lgx > a->w) {
+            if (std::max(w, a->w) * std::max(h, a->h) * sizeof(float) <= kAtlasMax) {
+                w = std::max(w, a->w);
+                h = std::max(h, a->h);
+            }
+            GF_CUDA(cudaEventSynchronize(a->used));  // the old one may still be read
+            a->drop();
+            if (a->make(w, h) != cudaSuccess) {
+                (void)cudaGetLastError();
+                a->drop();
+                return;
+            }
+            lay.lgx = lgx;
+        }
+        st = stream;
+        t = a;
+        t->busy = true;
+    }
+    ~AtlasUse()
+    {
+        if (!t) return;
+        std::lock_guard<std::mutex> g(kept_lock());
+        (void)cudaEventRecord(t->used, st);
+        t->busy = false;
+    }
+};
 
 template <typename T>
 static void project_t(genfire_ctx *ctx, const T *vol, int n1, int n2, int n3, long long vs1, long long vs2, int P,
                       const double *d_R, T *d_proj, const double *d_meas, double *d_sums, cudaStream_t st)
 {
     const long long npix = (long long)n1 * n2;
-    ProjTexture *at = nullptr;
+    AtlasUse at;
     if constexpr (sizeof(T) == 4) {
         // from 2^22 samples on: below, a call is bound by its launches and copies
         // (2^20 samples: 76 us with loads, 64 with gathers; 2^22: 106 and 92; 2^27:
-        // 1050 and 645), and the array of a volume size not seen before costs
-        // 0.1-0.2 ms once
-        if (ctx->interp == GENFIRE_INTERP_TRILINEAR && npix * n3 * P >= kTexSamples) at = atlas(ctx, n1, n2, n3);
+        // 1050 and 645), and an array, the first one or a larger one, costs 0.1-0.2 ms
+        // once
+        if (ctx->interp == GENFIRE_INTERP_TRILINEAR && npix * n3 * P >= kTexSamples)
+            at.take(ctx, n1, n2, n3, st);
     }
-    const unsigned nblk = at ? cdiv(n1, 16) * cdiv(n2, 16) : cdiv(npix, kProjThreads);
+    const unsigned nblk = at.t ? cdiv(n1, 16) * cdiv(n2, 16) : cdiv(npix, kProjThreads);
     DevBuf part;
     if (d_meas) part.alloc(sizeof(double) * 4 * (size_t)nblk * P, st);
     dim3 grid(nblk, P);
-    if (at) {
+    if (at.t) {
         if constexpr (sizeof(T) == 4) {
-            k_atlas_write<<<dim3(cdiv(npix, 256), n3), 256, 0, st>>>(vol, vs1, vs2, at->t, at->surf);
+            k_atlas_write<<<dim3(cdiv(npix, 256), n3), 256, 0, st>>>(vol, vs1, vs2, at.lay, at.t->surf);
             GF_CHECK_LAUNCH();
-            k_project_tex<<<grid, kProjThreads, 0, st>>>(at->tex, at->t, d_R, d_proj, d_meas, part.as<double>());
+            k_project_tex<<<grid, kProjThreads, 0, st>>>(at.t->tex, at.lay, d_R, d_proj, d_meas, part.as<double>());
         }
     } else if (ctx->interp == GENFIRE_INTERP_CUBIC)
         k_project<T, true><<<grid, kProjThreads, 0, st>>>(vol, n1, n2, n3, vs1, vs2, d_R, d_proj, d_meas,
