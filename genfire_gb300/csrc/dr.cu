@@ -28,6 +28,7 @@
 #include "internal.h"
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -574,12 +575,21 @@ static double pass_gain(int variant, int n)
     }
 }
 
-// 1 / N as a value and the rest of it, less the mean gain of the transforms
+// 1 / N less the mean gain of the transforms, as a value and the rest of it
 template <typename T> static void inverse_scale(RowPassArgs<T> &r, double N, double gain)
 {
-    const double s = (1.0 - gain) / N;
-    r.scale = (T)(1.0 / N);
-    r.scale_lo = (T)(s - (double)r.scale);
+    if constexpr (sizeof(T) == 8) {
+        r.scale = 1.0 / N;
+        r.scale_lo = 0;
+    } else {
+        // the value rounded down and the rest positive (never zero: a power of two's
+        // is far below the result's last place), so that both products of an
+        // infinite sum are infinities of its own sign
+        const double s = (1.0 - gain) / N;
+        r.scale = (float)s;
+        if ((double)r.scale > s) r.scale = std::nextafter(r.scale, 0.f);
+        r.scale_lo = std::max((float)(s - (double)r.scale), FLT_MIN);
+    }
 }
 
 static int round_up(int a, int b) { return (a + b - 1) / b * b; }

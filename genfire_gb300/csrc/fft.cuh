@@ -679,7 +679,7 @@ template <typename T> struct RowPassArgs {
     int positivity;
     cplx<T> *Y;        // ld1 x nrows half spectrum
     T scale;           // inverse only
-    T scale_lo;        // inverse, complex64: what scale misses of the exact factor
+    T scale_lo;        // inverse, complex64: what scale misses of the exact factor (positive)
     // with ctl set (the iteration's first pass): CTA 0 starts the iteration
     // (ctl_begin_update) while every CTA reads the object from xs[ctl->xnext]
     Ctl *ctl;
@@ -688,7 +688,8 @@ template <typename T> struct RowPassArgs {
 
 // a value times an inverse row pass's factor: one more multiply-add in FP32
 // gives it 48 bits, so that neither the rounding of 1/N nor the transforms' mean
-// gain (see pass_gain in dr.cu) scales the object at every iteration
+// gain (see pass_gain in dr.cu) scales the object at every iteration.  Both parts
+// are positive: an infinite sum stays infinite.
 __device__ __forceinline__ float scaled(float x, const RowPassArgs<float> &a) { return fmaf(x, a.scale, x * a.scale_lo); }
 __device__ __forceinline__ double scaled(double x, const RowPassArgs<double> &a) { return x * a.scale; }
 
