@@ -308,27 +308,62 @@ __device__ __forceinline__ void reg_fft(cplx<T> (&v)[NC][8], cplx<T> *sA, cplx<T
 // passes.
 template <typename T> using ErrAcc = typename std::conditional<sizeof(T) == 8, double, float>::type;
 
+// A sum of single-precision values kept as the unevaluated sum of two floats (48
+// bits and more), for the two-stage passes: their lengths' errK sums were FP64
+// before, and an FP64 pipe of 2 operations per clock per SM made their fused pass
+// 25 to 45 % slower (300 x 225 x 300 grid, a quarter of it measured: 97 us with FP32
+// sums, 101 with pairs, 129 with FP64; 450^3 484, 509, 605).  A term's difference
+// and every addition keep their rounding error (Knuth's two-sum).
+struct PairSum {
+    float hi, lo;
+};
+template <typename T> using ErrPair = typename std::conditional<sizeof(T) == 8, double, PairSum>::type;
+
+// s + e = a + b exactly, s the rounded sum
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
+{
+    s = __fadd_rn(a, b);
+    const float t = __fsub_rn(s, a);
+    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+}
+__device__ __forceinline__ void add_pair(PairSum &s, float hi, float lo)
+{
+    float h, e;
+    two_sum(s.hi, hi, h, e);
+    e = __fadd_rn(e, __fadd_rn(s.lo, lo));
+    if (e != e) e = 0.f;  // an infinite sum stays infinite, with a lo of NaN (h tells a NaN sum)
+    s.hi = __fadd_rn(h, e);
+    s.lo = __fadd_rn(__fsub_rn(h, s.hi), e);
+}
+// acc += |a - b|
+__device__ __forceinline__ void add_abs_diff(PairSum &acc, float a, float b)
+{
+    float d, e;
+    two_sum(a, -b, d, e);
+    add_pair(acc, fabsf(d), d < 0.f ? -e : e);
+}
+__device__ __forceinline__ void add_abs_diff(float &acc, float a, float b) { acc += fabsf(a - b); }
+__device__ __forceinline__ void add_abs_diff(double &acc, double a, double b) { acc += fabs(a - b); }
+
 // Fourier constraint and errK terms on one shared-memory tile (see k_colpass);
 // returns this thread's errK terms; idx maps (q3, column in tile) to the
 // tile's shared-memory slot.
-template <typename T, class Idx>
-__device__ __forceinline__ ErrAcc<T> apply_table_at(cplx<T> *s, const ColPassArgs<T> &a, int tile, int W, int other,
-                                                    Idx idx)
+template <typename T, class A_, class Idx>
+__device__ __forceinline__ A_ apply_table_at(cplx<T> *s, const ColPassArgs<T> &a, int tile, int W, int other, Idx idx)
 {
-    using A_ = ErrAcc<T>;
     const int cid0 = other * a.h1 + tile * W;
     const int cid1 = min(cid0 + W, other * a.h1 + a.h1);
     const int e0 = a.tab_off[cid0], e1 = a.tab_off[cid1];
     const int ci = *a.cidx;
-    A_ acc = 0;
+    A_ acc = {};
     for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
         const TabEntry<T> t = a.tab[e];
         const int q3 = t.pos & 0xFFFF, cl = t.pos >> 16;
         const int si = idx(q3, cl);
         const cplx<T> k = s[si];
-        const A_ mk_ = (A_)sqrt(k.x * k.x + k.y * k.y);
-        if (t.eflags & 1u) acc += fabs(mk_ - (A_)t.abs_q());
-        if (t.eflags & 2u) acc += fabs(mk_ - (A_)t.abs_mq());
+        const T mk_ = sqrt(k.x * k.x + k.y * k.y);
+        if (t.eflags & 1u) add_abs_diff(acc, mk_, t.abs_q());
+        if (t.eflags & 2u) add_abs_diff(acc, mk_, t.abs_mq());
         const bool eq = (t.cq >> ci) & 1u, emq = (t.cmq >> ci) & 1u;
         if (eq || emq) {
             const cplx<T> A = eq ? t.Mq : k;
@@ -341,17 +376,26 @@ __device__ __forceinline__ ErrAcc<T> apply_table_at(cplx<T> *s, const ColPassArg
 template <typename T, class Lay>
 __device__ __forceinline__ ErrAcc<T> apply_table(cplx<T> *s, const ColPassArgs<T> &a, int tile, int W, int other)
 {
-    return apply_table_at<T>(s, a, tile, W, other, [](int q3, int cl) { return Lay::idx(q3, cl); });
+    return apply_table_at<T, ErrAcc<T>>(s, a, tile, W, other, [](int q3, int cl) { return Lay::idx(q3, cl); });
 }
 
-// CTA sum of the per-thread errK terms: warp sums in FP32 (a few terms per
-// thread), the per-warp partials in FP64.  FP64 arithmetic is kept to one warp
-// because its throughput on this part is a small fraction of FP32's.
+// CTA sum of the per-thread errK terms: warp sums in the accumulator's own kind (FP32
+// for a few terms per thread, or pairs), the per-warp partials in FP64.  FP64
+// arithmetic is kept to one warp because its throughput on this part is a small
+// fraction of FP32's.
+template <typename A_> __device__ __forceinline__ void add_lane(A_ &acc, int o) { acc += __shfl_down_sync(0xffffffffu, acc, o); }
+__device__ __forceinline__ void add_lane(PairSum &acc, int o)
+{
+    const float hi = __shfl_down_sync(0xffffffffu, acc.hi, o), lo = __shfl_down_sync(0xffffffffu, acc.lo, o);
+    add_pair(acc, hi, lo);
+}
+template <typename A_> __device__ __forceinline__ double acc_value(A_ acc) { return (double)acc; }
+__device__ __forceinline__ double acc_value(PairSum acc) { return (double)acc.hi + (acc.lo != acc.lo ? 0.0 : (double)acc.lo); }
 template <typename A_> __device__ __forceinline__ void block_partial(A_ acc, double *out)
 {
     __shared__ double red[32];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (double)acc;
+    for (int o = 16; o > 0; o >>= 1) add_lane(acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc_value(acc);
     __syncthreads();
     if (threadIdx.x == 0) {
         double v = 0.0;

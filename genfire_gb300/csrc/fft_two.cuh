@@ -360,7 +360,7 @@ __device__ __forceinline__ void col_two(const ColPassArgs<T> &a, const Plan &tp,
             capture_rfree<T>(s, a, blockIdx.x, W, blockIdx.y, idx);
             __syncthreads();
         }
-        const ErrAcc<T> err = apply_table_at<T>(s, a, blockIdx.x, W, blockIdx.y, idx);
+        const ErrPair<T> err = apply_table_at<T, ErrPair<T>>(s, a, blockIdx.x, W, blockIdx.y, idx);
         block_partial(err, a.partial + (long long)blockIdx.y * gridDim.x + blockIdx.x);
         __syncthreads();
     }
