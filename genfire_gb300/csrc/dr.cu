@@ -292,10 +292,13 @@ template <typename T> static bool col_variant_ok(const ColPassArgs<T> &a, int v)
 // powers of two, two columns per thread in the fused forward + constraint +
 // inverse pass (two transforms per load) and one column per thread in the
 // single-transform passes (twice the resident warps); the mixed-radix
-// register engine for 3 or 5 times a power of two (the two-stage engine is
-// within 15 % of it either way there, and a candidate of the autotuner); the
-// two-stage engine for the other lengths that split (450 points, the fused
-// pass: 2.21 ms generic, 0.33 ms); the generic engine for the rest.
+// register engine for 3 or 5 times a power of two; the two-stage engine for the
+// other lengths that split (450 points, the fused pass: 2.21 ms generic, 0.33 ms)
+// and for the fused pass at five times a power of two (whole iterations of cubes,
+// complex64, F2 F3 I2 in us, mixed radix against two-stage: 320 points 33 261 35, 35
+// 155 37; 640 points 283 2073 281, 319 1245 288; three times one: 192 points 11.8
+// 35.3 12.8, 13.9 37.2 14.0; 384 points 53 272 63, 58 274 59; 768 points, a box of a
+// third, 316 1967 326, 377 2375 347); the generic engine for the rest.
 template <typename T> static int default_col_variant(const ColPassArgs<T> &a)
 {
     // below 512 points the radix-32 engine is a candidate of the autotuner, not
@@ -303,7 +306,8 @@ template <typename T> static int default_col_variant(const ColPassArgs<T> &a)
     // to 12.8 k iterations/s; as the default it cost the batched problems 1.5 %)
     if (a.pl.n >= 512 && col_variant_ok(a, kColR32)) return kColR32;
     if (reg_capable(a)) return ((a.mode & 3) == 3 && pair_capable(a)) ? kColReg2 : kColReg1;
-    if (col_variant_ok(a, kColMix)) return kColMix;
+    const bool five_fused = a.pl.n % 5 == 0 && (a.mode & 3) == 3;
+    if (col_variant_ok(a, kColMix) && !(five_fused && col_variant_ok(a, kColTwo))) return kColMix;
     if (col_variant_ok(a, kColTwo)) return kColTwo;
     return kColGeneric;
 }
@@ -414,10 +418,10 @@ template <typename T> static int autotune_colpass(ColPassArgs<T> a, int other, c
     float best_ms = 0, default_ms = -1;
     for (int v : {kColGeneric, kColReg1, kColReg2, kColMix, kColR32, kColR32Tma, kColTwo}) {
         if (!col_variant_ok(a, v)) continue;
-        // lengths whose engine is the two-stage one: the generic engine is near it
-        // only where a pass is one launch latency long, and choosing between them
-        // by time would give two processes different bits
-        if (v == kColGeneric && default_col_variant(a) == kColTwo) continue;
+        // the two-stage engine is the built-in choice or none: where it and another
+        // lie near each other, a choice by time would give two processes
+        // different bits
+        if ((v == kColTwo) != (default_col_variant(a) == kColTwo)) continue;
         launch_colpass<T>(a, other, st, v);
         GF_CUDA(cudaEventRecord(e0, st));
         for (int r = 0; r < 3; ++r) launch_colpass<T>(a, other, st, v);
