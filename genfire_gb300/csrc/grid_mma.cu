@@ -341,6 +341,15 @@ __device__ __forceinline__ bool ws_wait(uint64_t *bar, uint32_t parity, long lon
     }
 }
 
+// A bounded wait whose outcome every lane of the warp shares: the tensor-memory loads
+// after it are warp-collective, and when another role gives up, one lane may find the
+// barrier's phase complete and the next one the abort flag set.
+__device__ __forceinline__ bool ws_wait_warp(uint64_t *bar, uint32_t parity, long long limit, volatile int *abort_flag)
+{
+    const bool got = ws_wait(bar, parity, limit, abort_flag);
+    return __all_sync(0xffffffffu, got);
+}
+
 // two floats rounded to a packed pair of the 16-bit operand type (first at the
 // lower address), and the halves of such a pair back as floats (exact)
 template <bool F16> __device__ __forceinline__ uint32_t pack2(float a, float b)
@@ -681,7 +690,7 @@ __global__ void __launch_bounds__(umma::kWsThreads, 1) k_dft_tcgen05(WsArgs a)
                 next = a.units[i + 2];
                 if (row < next.nj) vnext = a.v[next.j0 + row];
             }
-            if (!ws_wait(&tfull[buf], (li >> 1) & 1, lim, abort_flag)) break;
+            if (!ws_wait_warp(&tfull[buf], (li >> 1) & 1, lim, abort_flag)) break;
             tc_fence_after();
             const uint32_t cre = tmem + lane_base + (uint32_t)(buf * 256), cim = cre + 128;
             float2 Fsum = make_float2(0.f, 0.f);
@@ -800,13 +809,6 @@ constexpr int kProdWarps = 8, kProdThreads = 32 * kProdWarps;
 constexpr int kWThreads = 32 * (kWProdWarp0 + kProdWarps);  // 544
 constexpr size_t kWSmem = (size_t)kWBBytes + (size_t)kWStages * kWAStage + 8 * kWNBars + 16;
 static_assert(kWSmem <= 227 * 1024, "shared memory of the N = 256 form");
-
-// a bounded wait whose outcome every lane of the warp shares
-__device__ __forceinline__ bool ws_wait_warp(uint64_t *bar, uint32_t parity, long long limit, volatile int *abort_flag)
-{
-    const bool got = ws_wait(bar, parity, limit, abort_flag);
-    return __all_sync(0xffffffffu, got);
-}
 }  // namespace umma
 
 template <bool F16, bool POW2>
