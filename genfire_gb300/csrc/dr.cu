@@ -1101,6 +1101,7 @@ template <typename T> struct ReconT : ReconBase {
     double denom = 0;
     int it_done = 0;
     int vF2 = kColAuto, vF3 = kColAuto, vI2 = kColAuto;  // column-pass variants (autotuned)
+    double gain = 0;                                     // of the passes' transforms (transform_gain)
     cudaGraphExec_t exec = nullptr;       // one iteration
     cudaGraphExec_t exec_long = nullptr;  // kLongGraph iterations, made by the first call that runs several of them
     std::vector<double> errR, Rarr, Rarr2;
@@ -1448,7 +1449,7 @@ template <typename T> struct ReconT : ReconBase {
         // every row is written
         q.pairmask = p.monitor_R == 1 ? nullptr : pairmask.as<uint8_t>();
         q.positivity = 0;
-        inverse_scale<T>(q, (double)n1 * n2 * n1, transform_gain());
+        inverse_scale<T>(q, (double)n1 * n2 * n1, gain);
         launch_rows<T>(q, false, st);
         mark();
     }
@@ -1529,7 +1530,14 @@ template <typename T> struct ReconT : ReconBase {
         return e;
     }
 
-    void build_graph() { exec = make_graph(1); }
+    // with the passes' engines settled; the gain is formed here, once: its hundreds
+    // of roots take longer on the host than a small grid's passes on the device,
+    // and stood between the launches when profile() enqueues them one by one
+    void build_graph()
+    {
+        gain = transform_gain();
+        exec = make_graph(1);
+    }
 
     // Rfree monitor (reconstruct.m:46-69, :137-146): withheld points of each
     // shell as 0-based linear indices into the centred grid; the caller has
