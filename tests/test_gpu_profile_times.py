@@ -1,8 +1,9 @@
-"""genfire_recon_profile's times of a small iteration are the passes' own: the host
-has no work to do between its launches that would pass for the last pass's time.
-On a 128^3 grid the row passes forward and back move the same bytes in a few
-microseconds each, and neither may show more than three times the others' longest
-(the inverse pass showed 60 microseconds and more when its factor was formed there)."""
+"""genfire_recon_profile's times are the passes' own: the host has no work to do
+between its launches that would pass for the last pass's time.  On grids of 4 x
+512 or 1024 x 4 points every pass is a launch latency long, and the last one may not
+show more than its bar times the others' longest (halfway, as a factor, between
+the 8 and 10 microseconds it takes and the 17 and 50 it showed when its factor was
+formed there, from the roots of unity of its 512 or 1024 points)."""
 import numpy as np
 import pytest
 
@@ -11,14 +12,13 @@ from tests.conftest import params
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("D,os_", [(64, 2.0), (50, 3.0)])
-def test_no_host_time_in_the_last_pass(lib, ctx, D, os_):
-    n = int(D * os_)
-    M = np.zeros((n, n, n), dtype=np.complex64, order="F")
-    M[:, :, ::4] = np.random.default_rng(D).random((n, n, 1))
-    r = ctx.recon(params(lib, D, D, 1, precision="mixed", oversamplingRatio=os_, numIterations=60), M)
+@pytest.mark.parametrize("D2,bar", [(256, 1.1), (512, 1.7)])
+def test_no_host_time_in_the_last_pass(lib, ctx, D2, bar):
+    M = np.zeros((4, 2 * D2, 4), dtype=np.complex64, order="F")
+    M[:, :, ::2] = np.random.default_rng(D2).random((4, 2 * D2, 1))
+    r = ctx.recon(params(lib, 2, D2, 1, precision="mixed", oversamplingRatio=2.0, numIterations=60), M)
     r.profile(10)
     ms = [r.profile(10)[1] for _ in range(5)]
     r.close()
     best = np.min(ms, axis=0)
-    assert best[-1] < 3 * best[:-1].max(), best
+    assert best[-1] < bar * best[:-1].max(), best
