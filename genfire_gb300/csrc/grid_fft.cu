@@ -12,6 +12,8 @@
 //                    shared memory, then FS = sum(w F) / sum(w) (:161) and
 //                    hermitianSymmetrize (:163, src/hermitianSymmetrize.m:22-65),
 //                    cast to the output precision: every voxel written once
+//                      (or k_fft_scatter and k_fft_finalize, the same by atomics
+//                    on the cube, where those are faster: scatter_faster)
 //   4. recIFFT         rec_ifft (dr.cu): My_stripzero(real(my_ifft(K))) (:165)
 //
 // Differences from the reference, by design: the sums are FP64 (the reference
@@ -77,6 +79,7 @@ struct __align__(16) FftSlice {
 };
 
 constexpr int kGatherThreads = 128;
+constexpr int kMerge = 4;  // lanes on one voxel from which a warp adds them up before the atomics
 constexpr int kMaxCube = 1290;  // the largest m with m^3 below 2^31
 constexpr size_t gather_smem(int m) { return sizeof(double) * 6 * (size_t)(2 * (m / 2) + 1); }
 
@@ -126,6 +129,11 @@ __device__ __forceinline__ float narrow(double x)
 // loop left each lane alone with its loads and atomics (3.56 ms).  One entry per
 // candidate, its samples added in registers first, measured 1.67 ms; a second
 // queue for a candidate's later pairs, which retry on the same voxel, 1.71.
+//
+// Where many of the 32 lie on one voxel (the axis of a tilt series, repeated
+// angles), the retries are a serial chain, and the lanes add up their values first:
+// 400 tilts of 48 x 48 (96^3 cube) 474 -> 302 us a call, one angle 100 times at 64 x
+// 64 291 -> 154, random angles unchanged (kMerge = 6: 310 and 155; 8: 333; 12: 385).
 template <typename T>
 __global__ void __launch_bounds__(kGatherThreads) k_fft_gather(const cplx<T> *__restrict__ X, const FftSlice *__restrict__ sl,
                                                                FftGridGeom g, unsigned long long *__restrict__ pairs,
@@ -152,26 +160,59 @@ __global__ void __launch_bounds__(kGatherThreads) k_fft_gather(const cplx<T> *__
     // sums the queue's first n (at most 32) pairs
     auto drain = [&](int n) {
         __syncwarp();
+        int k1 = 0;
+        double A[3] = {0.0, 0.0, 0.0}, B[3] = {0.0, 0.0, 0.0};  // w re, w im, w of the pair's two samples
         if (lane < n) {
             const uint2 q = qpos[warp][lane];
             const double wgt = widen(qw[warp][lane]);
-            const int k1 = (int)(q.x & 0xFFFFu) - h, p = (int)(q.x >> 16);
+            k1 = (int)(q.x & 0xFFFFu) - h;
+            const int p = (int)(q.x >> 16);
             const int i = (int)(q.y & 0xFFFFu) - h, j = (int)(q.y >> 16) - h;
             const cplx<T> *Xp = X + (size_t)p * m * m;
             const bool onA = inA && k1 <= hi && i <= hi && j <= hi;
             const bool onB = inB && !self && -k1 <= hi && -i <= hi && -j <= hi;
-            cplx<T> va = mk((T)0, (T)0), vb = va;
+            cplx<T> va = mk((T)-999, (T)0), vb = va;  // the reference's flag of a bad value
             if (onA) va = Xp[(i < 0 ? i + m : i) + (size_t)m * (j < 0 ? j + m : j)];
             if (onB) vb = Xp[(i > 0 ? m - i : -i) + (size_t)m * (j > 0 ? m - j : -j)];
-            auto add = [&](double *to, cplx<T> val) {
-                if (val.x == (T)-999 && val.y == (T)0) return;  // the reference's flag of a bad value
-                atomicAdd(to, widen(val.x) * wgt);
-                atomicAdd(to + L, widen(val.y) * wgt);
-                atomicAdd(to + 2 * L, wgt);
+            auto pair = [&](double (&v)[3], cplx<T> val) {
+                if (val.x == (T)-999 && val.y == (T)0) return;
+                v[0] = widen(val.x) * wgt;
+                v[1] = widen(val.y) * wgt;
+                v[2] = wgt;
                 ++cnt;
             };
-            if (onA) add(acc + k1 + h, va);
-            if (onB) add(acc + 3 * L + k1 + h, vb);
+            pair(A, va);
+            pair(B, vb);
+        }
+        // The lanes of one voxel, as a list: where one has kMerge of them, every list is
+        // summed into its first lane, which alone adds to the row (next: the lane
+        // whose partial sum continues this one's, or itself at the end).
+        const unsigned peers = __match_any_sync(0xffffffffu, lane < n ? k1 : m + lane);
+        bool first = lane < n;
+        if (__any_sync(0xffffffffu, __popc(peers) >= kMerge)) {
+            first = first && lane == __ffs(peers) - 1;
+            const unsigned above = lane == 31 ? 0u : peers & (0xffffffffu << (lane + 1));
+            int next = above ? __ffs(above) - 1 : lane;  // (lane itself: the end)
+            while (__any_sync(0xffffffffu, next != lane)) {
+                const bool more = next != lane;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const double a = __shfl_sync(0xffffffffu, A[c], next), b = __shfl_sync(0xffffffffu, B[c], next);
+                    if (more) {
+                        A[c] += a;
+                        B[c] += b;
+                    }
+                }
+                const int n2 = __shfl_sync(0xffffffffu, next, next);
+                next = more ? (n2 == next ? lane : n2) : lane;
+            }
+        }
+        if (first) {
+            double *to = acc + k1 + h;
+            if (A[2] > 0.0)
+                for (int c = 0; c < 3; ++c) atomicAdd(to + c * L, A[c]);
+            if (B[2] > 0.0)
+                for (int c = 0; c < 3; ++c) atomicAdd(to + (3 + c) * L, B[c]);
         }
         __syncwarp();
         if (lane < queued - n) {  // the rest (fewer than 32) moves to the front
@@ -301,6 +342,123 @@ __global__ void __launch_bounds__(kGatherThreads) k_fft_gather(const cplx<T> *__
     }
 }
 
+// The scatter: one thread per sample (x over the centred dim-1 index i, y = j, z =
+// projection), FP64 atomics on sums of the whole cube in global memory, which
+// k_fft_finalize averages and symmetrises.  Those atomics need no retries, but
+// the cube's sums, 24 bytes a voxel, are cleared, updated and read back.
+template <typename T>
+__global__ void __launch_bounds__(128) k_fft_scatter(const cplx<T> *__restrict__ X, const FftSlice *__restrict__ sl,
+                                                     FftGridGeom g, double2 *__restrict__ num,
+                                                     double *__restrict__ ws, unsigned long long *__restrict__ pairs)
+{
+    const int m = g.m, h = m / 2;
+    const int j = blockIdx.y, p = blockIdx.z;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned cnt = 0;
+    if (i < m) {
+        // centred (i, j) of my_fft = FFT index (i - h, j - h) mod m
+        const cplx<T> val = X[(size_t)p * m * m + wrap(i - h, m) + (size_t)m * wrap(j - h, m)];
+        if (!(val.x == (T)-999 && val.y == (T)0)) {
+            const float *r = sl[p].r;
+            const float kx = (float)(i - h), ky = (float)(j - h);
+            const float cx = __fadd_rn(__fmul_rn(r[0], kx), __fmul_rn(r[1], ky));
+            const float cy = __fadd_rn(__fmul_rn(r[2], kx), __fmul_rn(r[3], ky));
+            const float cz = __fadd_rn(__fmul_rn(r[4], kx), __fmul_rn(r[5], ky));
+            const float rx = roundf(cx), ry = roundf(cy), rz = roundf(cz);
+            for (int ys = -g.s; ys <= g.s; ++ys)
+                for (int xs = -g.s; xs <= g.s; ++xs)
+                    for (int zs = -g.s; zs <= g.s; ++zs) {
+                        const float tx = __fadd_rn(rx, (float)xs), ty = __fadd_rn(ry, (float)ys),
+                                    tz = __fadd_rn(rz, (float)zs);
+                        const int ix = (int)tx + h, iy = (int)ty + h, iz = (int)tz + h;
+                        if (ix < 0 || ix >= m || iy < 0 || iy >= m || iz < 0 || iz >= m) continue;
+                        const float dx = __fsub_rn(cx, tx), dy = __fsub_rn(cy, ty), dz = __fsub_rn(cz, tz);
+                        const float d = __fsqrt_rn(
+                            __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+                        if (!(d <= g.cut_le)) continue;
+                        const double w = (double)__fdiv_rn(1.0f, __fadd_rn(d, 1e-5f));
+                        const size_t v = (size_t)ix + (size_t)m * (iy + (size_t)m * iz);
+                        atomicAdd(&num[v].x, (double)val.x * w);
+                        atomicAdd(&num[v].y, (double)val.y * w);
+                        atomicAdd(&ws[v], w);
+                        ++cnt;
+                    }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(pairs, (unsigned long long)cnt);
+}
+
+// sum(w F) / sum(w) where sum(w) > 0, else 0: in FP64 for the FP64 output,
+// in FP32 from the FP64 sums for the single-precision output (no FP64
+// arithmetic: this part's FP64 pipe issues 2 operations per clock per SM).
+// The weight sum is >= 0, so it is positive iff its bits, as an integer, are.
+template <typename TO>
+__device__ __forceinline__ cplx<TO> fs_avg(const double2 *__restrict__ num, const double *__restrict__ ws, size_t v)
+{
+    cplx<TO> a = mk((TO)0, (TO)0);
+    if (reinterpret_cast<const long long *>(ws)[v] > 0) {
+        const double2 s = num[v];
+        if constexpr (sizeof(TO) == 8) {
+            const double w = ws[v];
+            a = mk(s.x / w, s.y / w);
+        } else {
+            const float w = (float)ws[v];
+            a = mk(__fdiv_rn((float)s.x, w), __fdiv_rn((float)s.y, w));
+        }
+    }
+    return a;
+}
+
+// grid: x over dim 1, y = dim-2 index, z = dim-3 index of the m^3 cube.
+// hermitianSymmetrize: mate of (i, j, k) is (e-1-i, e-1-j, e-1-k) on the
+// odd-extended cube (e = m + 1 for even m), zero beyond the input; the two
+// values are averaged over the number of non-zero ones.
+template <typename TO>
+__global__ void k_fft_finalize(const double2 *__restrict__ num, const double *__restrict__ ws, int m,
+                               cplx<TO> *__restrict__ M)
+{
+    const int j = blockIdx.y, k = blockIdx.z;
+    const int e = m + (m % 2 == 0);
+    const int mj = e - 1 - j, mk_ = e - 1 - k;
+    const size_t row = (size_t)m * (j + (size_t)m * k);
+    const size_t mrow = (size_t)m * (mj + (size_t)m * mk_);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+        const int mi = e - 1 - i;
+        const cplx<TO> a = fs_avg<TO>(num, ws, row + i);
+        cplx<TO> b = mk((TO)0, (TO)0);
+        if (mi < m && mj < m && mk_ < m) b = fs_avg<TO>(num, ws, mrow + mi);
+        TO re = a.x + b.x, im = a.y - b.y;
+        const int cnt = (a.x != 0 || a.y != 0) + (b.x != 0 || b.y != 0);
+        if (cnt == 2) { re *= (TO)0.5; im *= (TO)0.5; }
+        M[row + i] = mk(re, im);
+    }
+}
+
+// Which of the two.  The gather's sums cost more per pair (read, add, compare and
+// swap in shared memory, and the rows near the origin, which every projection
+// reaches, are few CTAs' work); the scatter's cost is the cube and the 27 or more
+// shifts tested per sample.  So the scatter is for many pairs per sample, and
+// for many projections of small ones.  us a call without recIFFT, complex64, random
+// angles, gather / scatter:
+//   cutoff 0.7, 100 projections: 64^3 103 / 88, 96^3 130 / 124, 128^3 142 / 178
+//   cutoff 0.3, 400 projections: 16^3 113 / 93, 64^3 135 / 133
+//   cutoff 1,    31 projections: 64^3 108 / 80, 128^3 137 / 141, 256^3 404 / 611
+//   cutoff 1.5,  31 projections: 128^3 264 / 202, 256^3 827 / 739; one: 256^3 131 / 218
+//   cutoff 3,    31 projections: 32^3 420 / 143, 128^3 1358 / 789; one: 32^3 105 / 124
+// The rule: 100 pairs or more per sample position, all projections together, of
+// cubes up to 48 + 16 times the pairs per sample (any size from 8 pairs on, which
+// one to three projections make up for only from 128 points on).  Shifts beyond 8
+// and windows wider than the cube stay with the gather, whose tests end at the
+// cube's and the slices' edges.
+static bool scatter_faster(int m, int P, int s, double cutoff)
+{
+    const double side = 2 * s + 1, c = std::max(cutoff, 0.0);
+    const double pairs = std::min(4.18879 * c * c * c, side * side * side);  // per sample
+    if (P * std::max(pairs, 0.5) < 100 || s > 8 || 2 * s >= m) return false;
+    return pairs >= 8 ? P >= 4 || m >= 128 : m <= 48 + 16 * pairs;
+}
+
 template <typename T>
 static void grid_fft_t(genfire_ctx *ctx, const genfire_params &p, const double *d_proj, const double *angles,
                        void *d_M, void *d_rec, int64_t *npairs)
@@ -340,7 +498,7 @@ static void grid_fft_t(genfire_ctx *ctx, const genfire_params &p, const double *
     DevBuf dsl(sizeof(FftSlice) * hs.size(), st), dpairs(sizeof(unsigned long long), st);
     GF_CUDA(cudaMemcpyAsync(dsl.p, hs.data(), sizeof(FftSlice) * hs.size(), cudaMemcpyHostToDevice, st));
     GF_CUDA(cudaMemsetAsync(dpairs.p, 0, sizeof(unsigned long long), st));
-    // 3: weighted averages and Hermitian symmetry, row pair by row pair
+    // 3: weighted averages and Hermitian symmetry
     FftGridGeom g;
     g.m = m;
     g.P = P;
@@ -350,11 +508,35 @@ static void grid_fft_t(genfire_ctx *ctx, const genfire_params &p, const double *
     // no pair is farther than its shift range and half a voxel allow
     const double reach = std::min(p.interpolationCutoffDistance, 1.7321 * (g.s + 0.5));
     g.reach = (float)reach + 0.01f;
-    const int h = m / 2;
-    raise_smem_limit(ctx->device, (const void *)k_fft_gather<T>, gather_smem(kMaxCube));
-    k_fft_gather<T><<<dim3(2 * h + 1, h + 1), kGatherThreads, gather_smem(m), st>>>(
-        X.as<cplx<T>>(), dsl.as<FftSlice>(), g, dpairs.as<unsigned long long>(), reinterpret_cast<cplx<T> *>(d_M));
+    bool scatter = scatter_faster(m, P, g.s, p.interpolationCutoffDistance);
+    DevBuf num, ws;
+    if (scatter) {
+        try {
+            num.alloc(sizeof(double2) * mm * m, st);
+            ws.alloc(sizeof(double) * mm * m, st);
+        } catch (const Error &e) {
+            if (e.st != GENFIRE_ERR_OOM) throw;
+            num.release();
+            scatter = false;  // the gather needs no sums of the cube
+        }
+    }
+    if (scatter) {
+        GF_CUDA(cudaMemsetAsync(num.p, 0, num.bytes, st));
+        GF_CUDA(cudaMemsetAsync(ws.p, 0, ws.bytes, st));
+        k_fft_scatter<T><<<dim3(cdiv(m, 128), m, P), 128, 0, st>>>(X.as<cplx<T>>(), dsl.as<FftSlice>(), g, num.as<double2>(),
+                                                                   ws.as<double>(), dpairs.as<unsigned long long>());
+        GF_CHECK_LAUNCH();
+        k_fft_finalize<T><<<dim3(cdiv(m, 256), m, m), 256, 0, st>>>(num.as<double2>(), ws.as<double>(), m,
+                                                                     reinterpret_cast<cplx<T> *>(d_M));
+    } else {
+        const int h = m / 2;
+        raise_smem_limit(ctx->device, (const void *)k_fft_gather<T>, gather_smem(kMaxCube));
+        k_fft_gather<T><<<dim3(2 * h + 1, h + 1), kGatherThreads, gather_smem(m), st>>>(
+            X.as<cplx<T>>(), dsl.as<FftSlice>(), g, dpairs.as<unsigned long long>(), reinterpret_cast<cplx<T> *>(d_M));
+    }
     GF_CHECK_LAUNCH();
+    num.release();
+    ws.release();
     X.release();
     // 4: recIFFT
     if (d_rec) rec_ifft(ctx, p.precision, d_M, m, m, D1, D2, d_rec);
