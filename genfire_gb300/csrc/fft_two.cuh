@@ -555,10 +555,21 @@ struct TwoFixed {
 };
 const TwoFixed *two_fixed(int n);  // nullptr: no kernel of its own
 
+// complex128 lengths up to 256 with a second factor above 16 and at least 1.5
+// times the first (125, 162, 200, 216, 243 and 250) stay with the generic engine:
+// the run-time kernels' 32 values a thread leave two CTAs per SM, and a third or
+// more of their threads are idle in the second stage.  An iteration of a cube, us,
+// two-stage / generic: 200 points 1751 / 1510, 216 points 1890 / 1740, 250 points 4389 /
+// 3239, and of the whole cube 125 points 1618 / 707, 243 points 6897 / 5164.  With a
+// factor of 7 the generic engine's butterfly is the slower one (252 points 3049 / 5669),
+// and above 256 points its passes are (270 points 3781 / 5987).
+inline bool two_unbalanced(const TwoPlan &p) { return p.N <= 256 && p.N % 7 && p.R2 > 16 && 2 * p.R2 >= 3 * p.R1; }
+
 template <typename T> bool two_capable(int n)
 {
     TwoPlan p;
-    return n <= 1024 && make_two_plan(n, p) && (sizeof(T) == 8 || p.R2 <= 16 || two_fixed(n));
+    if (n > 1024 || !make_two_plan(n, p)) return false;
+    return sizeof(T) == 8 ? !two_unbalanced(p) : p.R2 <= 16 || two_fixed(n);
 }
 
 // Mean gains (squared length, less 1) of complex64 arithmetic, from the rounding
