@@ -528,8 +528,15 @@ static void project_t(genfire_ctx *ctx, const T *vol, int n1, int n2, int n3, lo
         // from 2^22 samples on: below, a call is bound by its launches and copies
         // (2^20 samples: 76 us with loads, 64 with gathers; 2^22: 106 and 92; 2^27:
         // 1050 and 645), and an array, the first one or a larger one, costs 0.1-0.2 ms
-        // once
-        if (ctx->interp == GENFIRE_INTERP_TRILINEAR && npix * n3 * P >= kTexSamples)
+        // once.  Writing the volume into it pays from 5 projections on: along the axes
+        // and in tilt series the load kernel's lanes share lines, and it needs no copy
+        // (256^3, us a call, loads / texture: one projection along dim 3 541 / 607, two
+        // 587 / 636, four tilts 835 / 990, eight 1219 / 1219; two random angles 656 / 628).
+        // With few lines what counts is the length of one, which the texture's are
+        // clipped to (64 x 64 x 1024, one projection 310 / 184, along dim 3 553 / 536; 8 x 8
+        // x 20000, four projections 1960 / 106; 128 x 128 x 256, one tilt 251 / 263).
+        const bool pays = P >= 5 || npix * P < 1 << 14;
+        if (ctx->interp == GENFIRE_INTERP_TRILINEAR && npix * n3 * P >= kTexSamples && pays)
             at.take(ctx, n1, n2, n3, st);
     }
     const unsigned nblk = at.t ? cdiv(n1, 16) * cdiv(n2, 16) : cdiv(npix, kProjThreads);
