@@ -248,12 +248,18 @@ __global__ void __launch_bounds__(mix_threads<T, N2, N1>()) k_row_c2r_mix(RowPas
 // ---------------------------------------------------------------------------
 // dispatch
 // ---------------------------------------------------------------------------
+// complex64 rows of up to 1024 points take the two-stage kernels (launch_rows in
+// dr.cu), so only the longer ones have row kernels here
+template <typename T> constexpr bool mix_rows(int n) { return sizeof(T) == 8 || n > 1024; }
+
 template <typename T, int N2, int N1> static void mix_attrs()
 {
     const int sm = (int)mix_smem<T, N2, N1>();
     GF_CUDA(cudaFuncSetAttribute((const void *)k_col_mix<T, N2, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    GF_CUDA(cudaFuncSetAttribute((const void *)k_row_r2c_mix<T, N2, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    GF_CUDA(cudaFuncSetAttribute((const void *)k_row_c2r_mix<T, N2, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    if constexpr (mix_rows<T>(N1 * N2)) {
+        GF_CUDA(cudaFuncSetAttribute((const void *)k_row_r2c_mix<T, N2, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        GF_CUDA(cudaFuncSetAttribute((const void *)k_row_c2r_mix<T, N2, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    }
 }
 
 template <typename T> static void ensure_mix_attrs()
@@ -326,15 +332,15 @@ template <typename T> bool launch_rows_mix(const RowPassArgs<T> &a, bool forward
 {
     int N1 = 0;
     const int N2 = mix_split<T>(a.pl.n, N1);
-    if (!N2) return false;
+    if (!N2 || !mix_rows<T>(a.pl.n)) return false;
     if (a.W != mix_width<T>(a.pl.n)) fail(GENFIRE_ERR_STATE, "internal: mixed-radix tile width mismatch.");
     ensure_mix_attrs<T>();
     const dim3 grid(cdiv((a.nrows + 1) / 2, a.W));
 #define GF_ROW(n2, n1)                                                                                    \
-    do {                                                                                                  \
+    if constexpr (mix_rows<T>(n1 * n2)) {                                                                 \
         if (forward) launch_pass(k_row_r2c_mix<T, n2, n1>, grid, mix_threads<T, n2, n1>(), mix_smem<T, n2, n1>(), st, a); \
         else launch_pass(k_row_c2r_mix<T, n2, n1>, grid, mix_threads<T, n2, n1>(), mix_smem<T, n2, n1>(), st, a);  \
-    } while (0)
+    }
     GF_MIX_CASES(GF_ROW)
 #undef GF_ROW
     return false;
