@@ -1097,7 +1097,7 @@ struct ReconBase {
 };
 
 // iterations of the long graph, and the count of a call from which it is made
-// (making it costs 0.2 ms, a launch of its own per iteration 3 us)
+// (making it costs 0.1 ms, a launch of its own per iteration 2 to 3 us)
 constexpr int kLongGraph = 4, kLongGraphFrom = 96;
 
 template <typename T> struct ReconT : ReconBase {
@@ -1688,8 +1688,7 @@ template <typename T> struct ReconT : ReconBase {
         cudaStream_t st = ctx->stream;
         // kLongGraph iterations per launch where as many are left before the next
         // stop (the R-factor monitor's): a launch of its own per iteration leaves a
-        // gap between them (200 iterations of a 64^3 object: 5.29 ms, 4.69 with the
-        // passes overlapped as well; see launch_pass)
+        // gap between them (figures at PassOverlap)
         const int stop = p.monitor_R == 1 ? p.monitorR_loopLength : 0;
         for (int left = count; left > 0;) {
             const int run = stop ? std::min(left, stop - it_done % stop) : left;

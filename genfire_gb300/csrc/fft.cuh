@@ -435,7 +435,8 @@ static __device__ __noinline__ void ctl_mid_update(Ctl *c, const double *partial
 // launch_pass under a PassOverlap, its launch is prepared while the pass before
 // it in the stream still runs, and its CTAs wait in pass_begin until that one has
 // completed and its writes are visible.  Nothing of the order changes, only the
-// launch latency goes: 200 iterations of a 64^3 object 5.08 -> 4.86 ms.  Used for
+// launch latency goes: 200 iterations of a 64^3 object take 4.94 ms with one graph
+// launch each, 4.52 with four per launch, 4.32 with this as well.  Used for
 // the long graphs only: in a graph of one iteration, launched again and again,
 // the edges cost as much as they gain (128^3 object, 50 iterations: 3.99 ms
 // without, 4.05 with).  Letting the next pass's CTAs come up early

@@ -1247,11 +1247,12 @@ void raise_smem_limit(int device, const void *kern, size_t bytes)
 // Which tensor-core DFT: the first form (N = 128, 128-point tiles) by default;
 // GENFIRE_DFT_KERNEL=n256 selects the second (Re and Im stacked in rows,
 // N = 256, 64-point tiles).  On 256 x 256 projections (90 of them, 2.77 M
-// points) the first takes 1.63 ms and the second 1.80 ms: the second's MMAs
-// alone run in 1.15 ms against the first's 1.31 ms (fewer shared-memory bytes
-// per MAC), but its K split (blocks of 128 rows) and row-wise Re/Im double the
-// E_v contraction twice over.  The choice is a fixed rule, not a timing, so
-// that a gridding call gives the same bits in every process (the two forms
+// points) the first takes 0.82 ms, folded over the rows, and the second, which
+// is not, 1.80 ms; before the fold the first took 1.63, the second's MMAs alone
+// running in 1.15 ms against 1.31 (fewer shared-memory bytes per MAC), but its K
+// split (blocks of 128 rows) and row-wise Re/Im doubling the E_v contraction twice
+// over.  The choice is a fixed rule, not a timing, so that a gridding call gives
+// the same bits in every process (the two forms
 // round differently).
 static bool dft_use_wide()
 {

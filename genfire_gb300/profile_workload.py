@@ -10,8 +10,8 @@ positivity and the ellipsoid support.
     python -m genfire_gb300.profile_workload project [calls]
         the MIXED R-factor of the ground-truth volume against the projections
         (k_project<float, trilinear> with the fused sums)
-    python -m genfire_gb300.profile_workload fftgrid [calls]
-        fillInFourierGrid (griddingMethod 1) calls, MIXED
+    python -m genfire_gb300.profile_workload fftgrid [calls] [cutoff]
+        fillInFourierGrid (griddingMethod 1) calls, MIXED (cutoff 0.125; the class default is 0.7)
 
 The workload's projections are made by the FP64 projector (three launches of
 k_project<double>) before the case runs.
@@ -87,6 +87,7 @@ def main(argv):
         calls = int(argv[1]) if len(argv) > 1 else 2
         p = _params(G, w, G.PREC_MIXED)
         p.griddingMethod = 1
+        p.interpolationCutoffDistance = float(argv[2]) if len(argv) > 2 else 0.125
         p.allowMultipleGridMatches = 1
         for _ in range(calls):
             t0 = time.time()
