@@ -130,11 +130,12 @@ __device__ __forceinline__ float narrow(double x)
 // candidate, its samples added in registers first, measured 1.67 ms; a second
 // queue for a candidate's later pairs, which retry on the same voxel, 1.71.
 //
-// Where many of the 32 lie on one voxel (the axis of a tilt series, repeated
+// MERGE: where many of the 32 lie on one voxel (the axis of a tilt series, repeated
 // angles), the retries are a serial chain, and the lanes add up their values first:
-// 400 tilts of 48 x 48 (96^3 cube) 474 -> 302 us a call, one angle 100 times at 64 x
-// 64 291 -> 154, random angles unchanged (kMerge = 6: 310 and 155; 8: 333; 12: 385).
-template <typename T>
+// 400 tilts of 48 x 48 (96^3 cube) 464 -> 301 us a call, one angle 100 times at 64 x
+// 64 293 -> 153 (kMerge = 6: 310 and 155; 8: 333; 12: 385).  With random angles
+// finding those lanes costs more than it saves (192^3 cube, 80 projections 228 -> 238).
+template <typename T, bool MERGE>
 __global__ void __launch_bounds__(kGatherThreads) k_fft_gather(const cplx<T> *__restrict__ X, const FftSlice *__restrict__ sl,
                                                                FftGridGeom g, unsigned long long *__restrict__ pairs,
                                                                cplx<T> *__restrict__ M)
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_fft_gather(const cplx<T> *__
     auto drain = [&](int n) {
         __syncwarp();
         int k1 = 0;
-        double A[3] = {0.0, 0.0, 0.0}, B[3] = {0.0, 0.0, 0.0};  // w re, w im, w of the pair's two samples
+        double A[3] = {0.0, 0.0, 0.0}, B[3] = {0.0, 0.0, 0.0};  // MERGE: w re, w im, w of the pair's two samples
         if (lane < n) {
             const uint2 q = qpos[warp][lane];
             const double wgt = widen(qw[warp][lane]);
@@ -171,48 +172,57 @@ __global__ void __launch_bounds__(kGatherThreads) k_fft_gather(const cplx<T> *__
             const cplx<T> *Xp = X + (size_t)p * m * m;
             const bool onA = inA && k1 <= hi && i <= hi && j <= hi;
             const bool onB = inB && !self && -k1 <= hi && -i <= hi && -j <= hi;
-            cplx<T> va = mk((T)-999, (T)0), vb = va;  // the reference's flag of a bad value
+            cplx<T> va = mk((T)0, (T)0), vb = va;
             if (onA) va = Xp[(i < 0 ? i + m : i) + (size_t)m * (j < 0 ? j + m : j)];
             if (onB) vb = Xp[(i > 0 ? m - i : -i) + (size_t)m * (j > 0 ? m - j : -j)];
-            auto pair = [&](double (&v)[3], cplx<T> val) {
-                if (val.x == (T)-999 && val.y == (T)0) return;
-                v[0] = widen(val.x) * wgt;
-                v[1] = widen(val.y) * wgt;
-                v[2] = wgt;
+            auto add = [&](double *to, double (&v)[3], cplx<T> val) {
+                if (val.x == (T)-999 && val.y == (T)0) return;  // the reference's flag of a bad value
+                if constexpr (MERGE) {
+                    v[0] = widen(val.x) * wgt;
+                    v[1] = widen(val.y) * wgt;
+                    v[2] = wgt;
+                } else {
+                    atomicAdd(to, widen(val.x) * wgt);
+                    atomicAdd(to + L, widen(val.y) * wgt);
+                    atomicAdd(to + 2 * L, wgt);
+                }
                 ++cnt;
             };
-            pair(A, va);
-            pair(B, vb);
+            if (onA) add(acc + k1 + h, A, va);
+            if (onB) add(acc + 3 * L + k1 + h, B, vb);
         }
-        // The lanes of one voxel, as a list: where one has kMerge of them, every list is
-        // summed into its first lane, which alone adds to the row (next: the lane
-        // whose partial sum continues this one's, or itself at the end).
-        const unsigned peers = __match_any_sync(0xffffffffu, lane < n ? k1 : m + lane);
-        bool first = lane < n;
-        if (__any_sync(0xffffffffu, __popc(peers) >= kMerge)) {
-            first = first && lane == __ffs(peers) - 1;
-            const unsigned above = lane == 31 ? 0u : peers & (0xffffffffu << (lane + 1));
-            int next = above ? __ffs(above) - 1 : lane;  // (lane itself: the end)
-            while (__any_sync(0xffffffffu, next != lane)) {
-                const bool more = next != lane;
+        if constexpr (MERGE) {
+            // the lanes of one voxel as a list, which is summed into its first lane, and
+            // that alone adds to the row (next: the lane whose partial sum continues this
+            // one's, or itself at the end)
+            const unsigned peers = __match_any_sync(0xffffffffu, lane < n ? k1 : m + lane);
+            bool first = lane < n;
+            if (__any_sync(0xffffffffu, __popc(peers) >= kMerge)) {
+                first = first && lane == __ffs(peers) - 1;
+                const unsigned above = lane == 31 ? 0u : peers & (0xffffffffu << (lane + 1));
+                int next = above ? __ffs(above) - 1 : lane;
+                while (__any_sync(0xffffffffu, next != lane)) {
+                    const bool more = next != lane;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const double a = __shfl_sync(0xffffffffu, A[c], next), b = __shfl_sync(0xffffffffu, B[c], next);
-                    if (more) {
-                        A[c] += a;
-                        B[c] += b;
+                    for (int c = 0; c < 3; ++c) {
+                        const double a = __shfl_sync(0xffffffffu, A[c], next), b = __shfl_sync(0xffffffffu, B[c], next);
+                        if (more) {
+                            A[c] += a;
+                            B[c] += b;
+                        }
                     }
+                    const int n2 = __shfl_sync(0xffffffffu, next, next);
+                    next = more ? (n2 == next ? lane : n2) : lane;
                 }
-                const int n2 = __shfl_sync(0xffffffffu, next, next);
-                next = more ? (n2 == next ? lane : n2) : lane;
             }
-        }
-        if (first) {
-            double *to = acc + k1 + h;
-            if (A[2] > 0.0)
-                for (int c = 0; c < 3; ++c) atomicAdd(to + c * L, A[c]);
-            if (B[2] > 0.0)
-                for (int c = 0; c < 3; ++c) atomicAdd(to + (3 + c) * L, B[c]);
+            if (first) {
+                double *to = acc + k1 + h;
+                // (a weight is positive, and told by its bits: no FP64 compare)
+                if (__double2hiint(A[2]))
+                    for (int c = 0; c < 3; ++c) atomicAdd(to + c * L, A[c]);
+                if (__double2hiint(B[2]))
+                    for (int c = 0; c < 3; ++c) atomicAdd(to + (3 + c) * L, B[c]);
+            }
         }
         __syncwarp();
         if (lane < queued - n) {  // the rest (fewer than 32) moves to the front
@@ -435,7 +445,26 @@ __global__ void k_fft_finalize(const double2 *__restrict__ num, const double *__
     }
 }
 
-// Which of the two.  The gather's sums cost more per pair (read, add, compare and
+// Whether many samples of a voxel come from different slices: the slices share an
+// axis or a plane.  With N the mean of n n' over the slices' unit normals, an
+// eigenvalue of N is then near zero (its determinant), or two are (the sum of its
+// principal 2 x 2 minors).  The first needs many slices to make up for MERGE (100 tilts of
+// 96 x 96: 288 -> 276 us, 31 of 64 x 64 no gain), of the second few do.
+static bool shared_axis(const std::vector<FftSlice> &sl)
+{
+    double N[6] = {0, 0, 0, 0, 0, 0};  // xx, yy, zz, xy, xz, yz
+    for (const FftSlice &f : sl) {
+        const double x = f.n[0], y = f.n[1], z = f.n[2];
+        N[0] += x * x; N[1] += y * y; N[2] += z * z;
+        N[3] += x * y; N[4] += x * z; N[5] += y * z;
+    }
+    for (double &v : N) v /= (double)sl.size();
+    const double minors = N[0] * N[1] - N[3] * N[3] + N[0] * N[2] - N[4] * N[4] + N[1] * N[2] - N[5] * N[5];
+    const double det = N[0] * (N[1] * N[2] - N[5] * N[5]) - N[3] * (N[3] * N[2] - N[5] * N[4]) + N[4] * (N[3] * N[5] - N[1] * N[4]);
+    return (sl.size() >= 96 && det < 1e-3) || (sl.size() >= 16 && minors < 0.01);
+}
+
+// Scatter or gather.  The gather's sums cost more per pair (read, add, compare and
 // swap in shared memory, and the rows near the origin, which every projection
 // reaches, are few CTAs' work); the scatter's cost is the cube and the 27 or more
 // shifts tested per sample.  So the scatter is for many pairs per sample, and
@@ -530,8 +559,9 @@ static void grid_fft_t(genfire_ctx *ctx, const genfire_params &p, const double *
                                                                      reinterpret_cast<cplx<T> *>(d_M));
     } else {
         const int h = m / 2;
-        raise_smem_limit(ctx->device, (const void *)k_fft_gather<T>, gather_smem(kMaxCube));
-        k_fft_gather<T><<<dim3(2 * h + 1, h + 1), kGatherThreads, gather_smem(m), st>>>(
+        const auto gather = shared_axis(hs) ? k_fft_gather<T, true> : k_fft_gather<T, false>;
+        raise_smem_limit(ctx->device, (const void *)gather, gather_smem(kMaxCube));
+        gather<<<dim3(2 * h + 1, h + 1), kGatherThreads, gather_smem(m), st>>>(
             X.as<cplx<T>>(), dsl.as<FftSlice>(), g, dpairs.as<unsigned long long>(), reinterpret_cast<cplx<T> *>(d_M));
     }
     GF_CHECK_LAUNCH();

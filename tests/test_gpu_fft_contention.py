@@ -26,6 +26,7 @@ def _angles(kind, P, rng):
     (8, 2.0, 69, 0.7, 1, "euler"), (8, 2.0, 70, 0.7, 1, "euler"), (8, 2.0, 199, 0.3, 1, "euler"), (8, 2.0, 200, 0.3, 1, "euler"),
     (9, 1.0, 100, 0.9, 0, "euler"), (9, 1.0, 99, 0.9, 0, "euler"), (6, 1.5, 24, 1.0, 1, "euler"), (9, 1.75, 8, 1.5, 1, "tilt"),
     (8, 2.0, 3, 2.4, 1, "euler"), (8, 2.0, 4, 2.4, 1, "same"), (5, 1.0, 40, 1.6, 1, "euler"), (4, 1.0, 40, 1.6, 1, "euler"),
+    (36, 2.0, 96, 0.7, 1, "tilt"), (10, 2.0, 100, 0.3, 1, "tilt"), (10, 2.0, 95, 0.3, 1, "tilt"), (10, 2.0, 16, 0.7, 1, "same"), (10, 2.0, 15, 0.7, 1, "same"),
     (10, 2.0, 60, 0.7, 1, "same"), (10, 2.0, 60, 0.7, 1, "tilt"), (24, 2.0, 90, 0.7, 1, "tilt"), (12, 2.0, 4, 9.0, 1, "euler")])
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_results(lib, ctx, oracle, D, os_, P, cut, am, kind, precision):
