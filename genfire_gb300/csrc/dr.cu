@@ -435,6 +435,10 @@ template <typename T> static int autotune_colpass(ColPassArgs<T> a, int other, c
         // lie near each other, a choice by time would give two processes
         // different bits
         if ((v == kColTwo) != (standard == kColTwo)) continue;
+        // at 128 points the radix-32 engine is as fast as the others when timed alone, but
+        // slower in the iteration (200 of a 64^3 object: 5.24 ms, 4.42 with one column per
+        // thread) and less exact (4.4e-6 against 2.5e-6 of the object after them)
+        if (v == kColR32 && a.pl.n < 256) continue;
         launch_colpass<T>(a, other, st, v);
         const float ms = timed(v, 3);
         if (v == standard) default_ms = ms;
