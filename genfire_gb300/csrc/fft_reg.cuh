@@ -312,8 +312,10 @@ template <typename T> using ErrAcc = typename std::conditional<sizeof(T) == 8, d
 // bits and more), for the two-stage passes: their lengths' errK sums were FP64
 // before, and an FP64 pipe of 2 operations per clock per SM made their fused pass
 // 25 to 45 % slower (300 x 225 x 300 grid, a quarter of it measured: 97 us with FP32
-// sums, 101 with pairs, 129 with FP64; 450^3 484, 509, 605).  A term's difference
-// and every addition keep their rounding error (Knuth's two-sum).
+// sums, 129 with FP64; 450^3 484 and 605).  A term's difference and every addition
+// keep their rounding error (Knuth's two-sum): 50 iterations of a 100 x 75 x 100
+// object on the first grid 6.51 ms with FP32 sums, 6.63 with pairs, 6.77 with the
+// pair normalised after each term.
 struct PairSum {
     float hi, lo;
 };
@@ -335,12 +337,18 @@ __device__ __forceinline__ void add_pair(PairSum &s, float hi, float lo)
     s.hi = __fadd_rn(h, e);
     s.lo = __fadd_rn(__fsub_rn(h, s.hi), e);
 }
-// acc += |a - b|
+// acc += |a - b| for magnitudes (not negative): the larger less the smaller and what
+// that rounds off, exact by the order of the two; the rounding errors gather in lo,
+// which the sum over the lanes carries over (a NaN fails the comparison and stays)
 __device__ __forceinline__ void add_abs_diff(PairSum &acc, float a, float b)
 {
-    float d, e;
-    two_sum(a, -b, d, e);
-    add_pair(acc, fabsf(d), d < 0.f ? -e : e);
+    const bool less = a < b;
+    const float big = less ? b : a, small = less ? a : b;
+    const float d = __fsub_rn(big, small), e = __fsub_rn(__fsub_rn(big, d), small);
+    float h, r;
+    two_sum(acc.hi, d, h, r);
+    acc.hi = h;
+    acc.lo = __fadd_rn(acc.lo, __fadd_rn(r, e));
 }
 __device__ __forceinline__ void add_abs_diff(float &acc, float a, float b) { acc += fabsf(a - b); }
 __device__ __forceinline__ void add_abs_diff(double &acc, double a, double b) { acc += fabs(a - b); }
