@@ -15,9 +15,10 @@
  *   - A context owns one CUDA stream on one device.  A context is not
  *     thread-safe; use one context per host thread.
  *   - Between calls a context keeps its projector's texture (up to 1 GiB, after
- *     the first single-precision trilinear projector call of 2^22 samples).  It
- *     is freed by genfire_destroy, and when an allocation of any context on the
- *     device fails.
+ *     the first single-precision trilinear projector call of 2^22 samples and
+ *     five projections, or of fewer where they are few long lines).  It is freed
+ *     by genfire_destroy, and when an allocation of any context on the device
+ *     fails.
  *   - Host-pointer entry points copy inputs to the device and results back.
  *     The *_device variants take device pointers (e.g. from cudaMalloc or a
  *     torch tensor) and leave results on the device.
