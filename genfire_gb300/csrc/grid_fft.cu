@@ -448,9 +448,11 @@ __global__ void k_fft_finalize(const double2 *__restrict__ num, const double *__
 // Whether many samples of a voxel come from different slices: the slices share an
 // axis or a plane.  With N the mean of n n' over the slices' unit normals, an
 // eigenvalue of N is then near zero (its determinant), or two are (the sum of its
-// principal 2 x 2 minors).  The first needs many slices to make up for MERGE (100 tilts of
-// 96 x 96: 288 -> 276 us, 31 of 64 x 64 no gain), of the second few do.
-static bool shared_axis(const std::vector<FftSlice> &sl)
+// principal 2 x 2 minors).  Of the first it takes many slices for the size of the cube
+// to make up for MERGE, of the second few do.  us a call without MERGE / with it,
+// complex64, tilt series: 100 on a 128^3 cube, cutoff 0.7 168 / 149, 0.2 92.6 / 92.3; 120 on
+// 200^3 358 / 331, 170 / 175; 100 on 320^3 727 / 718, 341 / 356.
+static bool shared_axis(const std::vector<FftSlice> &sl, int m)
 {
     double N[6] = {0, 0, 0, 0, 0, 0};  // xx, yy, zz, xy, xz, yz
     for (const FftSlice &f : sl) {
@@ -461,7 +463,7 @@ static bool shared_axis(const std::vector<FftSlice> &sl)
     for (double &v : N) v /= (double)sl.size();
     const double minors = N[0] * N[1] - N[3] * N[3] + N[0] * N[2] - N[4] * N[4] + N[1] * N[2] - N[5] * N[5];
     const double det = N[0] * (N[1] * N[2] - N[5] * N[5]) - N[3] * (N[3] * N[2] - N[5] * N[4]) + N[4] * (N[3] * N[5] - N[1] * N[4]);
-    return (sl.size() >= 96 && det < 1e-3) || (sl.size() >= 16 && minors < 0.01);
+    return (sl.size() >= 96 && 4 * sl.size() >= 3 * (size_t)m && det < 1e-3) || (sl.size() >= 16 && minors < 0.01);
 }
 
 // Scatter or gather.  The gather's sums cost more per pair (read, add, compare and
@@ -559,7 +561,7 @@ static void grid_fft_t(genfire_ctx *ctx, const genfire_params &p, const double *
                                                                      reinterpret_cast<cplx<T> *>(d_M));
     } else {
         const int h = m / 2;
-        const auto gather = shared_axis(hs) ? k_fft_gather<T, true> : k_fft_gather<T, false>;
+        const auto gather = shared_axis(hs, m) ? k_fft_gather<T, true> : k_fft_gather<T, false>;
         raise_smem_limit(ctx->device, (const void *)gather, gather_smem(kMaxCube));
         gather<<<dim3(2 * h + 1, h + 1), kGatherThreads, gather_smem(m), st>>>(
             X.as<cplx<T>>(), dsl.as<FftSlice>(), g, dpairs.as<unsigned long long>(), reinterpret_cast<cplx<T> *>(d_M));
